@@ -1373,7 +1373,7 @@ extern "C" int qx_grad_adjoint_jvp(qx_handle* h, const double* D, double cj, dou
 
 // ------------------------------------------------------ one-electron integrals --
 void qx_launch_oei(const qx::PairInfo* pairs, int npair, const qx::PrimPair* prims, const double* boys,
-                   const double* xyz, const double* Z, int natom, long long n, double* S, double* T, double* V,
+                   const double* rys, const double* xyz, const double* Z, int natom, long long n, double* S, double* T, double* V,
                    double* dS, double* dT, double* dV, cudaStream_t s);
 
 extern "C" int qx_set_charges(qx_handle* h, const double* Z) {
@@ -1398,7 +1398,7 @@ extern "C" int qx_oei(qx_handle* h, double* S, double* T, double* V, void* strea
     if (!h) return fail(QX_E_INVALID, "qx_oei: NULL handle");
     if (!h->d_Z) return fail(QX_E_INVALID, "qx_oei: nuclear charges not set (qx_set_charges)");
     DeviceGuard g(h->device);
-    qx_launch_oei(h->d_pairs, (int)h->pairs.size(), h->d_prims, h->d_boys, h->d_xyz, h->d_Z, h->natom, h->nbf, S, T,
+    qx_launch_oei(h->d_pairs, (int)h->pairs.size(), h->d_prims, h->d_boys, h->d_rys, h->d_xyz, h->d_Z, h->natom, h->nbf, S, T,
                   V, nullptr, nullptr, nullptr, (cudaStream_t)stream);
     QX_CUDA(cudaGetLastError());
     return QX_OK;
@@ -1414,7 +1414,7 @@ extern "C" int qx_oei_deriv_core(qx_handle* h, int order, double* dS, double* dT
     QX_CUDA(cudaMemsetAsync(dS, 0, bytes, s));
     QX_CUDA(cudaMemsetAsync(dT, 0, bytes, s));
     QX_CUDA(cudaMemsetAsync(dV, 0, bytes, s));
-    qx_launch_oei(h->d_pairs, (int)h->pairs.size(), h->d_prims, h->d_boys, h->d_xyz, h->d_Z, h->natom, h->nbf,
+    qx_launch_oei(h->d_pairs, (int)h->pairs.size(), h->d_prims, h->d_boys, h->d_rys, h->d_xyz, h->d_Z, h->natom, h->nbf,
                   nullptr, nullptr, nullptr, dS, dT, dV, s);
     QX_CUDA(cudaGetLastError());
     return QX_OK;

@@ -40,6 +40,24 @@ def test_oei_matches_host(case):
         assert np.abs(d.reshape(-1, 3, *d.shape[1:]).sum(axis=0)).max() < 1e-10
 
 
+@pytest.mark.parametrize("natom,charges,f", [(1, (8,), True), (2, (6, 8), True), (9, (1,), False)])
+def test_oei_nuclear_slices(natom, charges, f):
+    """A lone atom (the Hermite form), two heavy atoms with every pair class up to
+    (f|f), and enough pairs that the nuclei are cut into unequal slices (9 atoms, 378
+    pairs: slices of 2 and a last one of 1)."""
+    from quax_b200.integrals.engine import EriEngine
+
+    spec = SyntheticSpec(natom=natom, box=6.0, min_sep=1.2, kmax=2, exp_lo=0.1, exp_hi=50.0, charges=charges,
+                         heavy_ls=(0, 1, 2), f_shell=f, f_kmax=1)
+    m, b = synthetic_molecule(spec, 3)
+    eng = EriEngine(b, 1e-12)
+    eng.set_charges(m.Z)
+    got = [x.cpu().numpy() for x in (*eng.oei(), *eng.oei_deriv(1))]
+    ref = one_electron(b, m.Z, b.atom_coords(), deriv=True)
+    for k, (g, h) in enumerate(zip(got, ref)):
+        assert np.abs(g - h).max() < (1e-12 if k < 3 else 1e-11) * max(1.0, np.abs(h).max()), k
+
+
 def test_oei_deriv_finite_differences():
     from quax_b200.integrals.engine import EriEngine
 
