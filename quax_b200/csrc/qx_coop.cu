@@ -60,8 +60,8 @@ __global__ void __launch_bounds__(COOP_WPB * 32) k_coop(CoopArgs ca, int mode) {
     double* V = coop_sm + (size_t)warp * C.vslots;
     double* accw = coop_sm + vreg + (size_t)warp * C.nacc;
     double* coef = coop_sm + vreg + (size_t)COOP_WPB * C.nacc + warp * 24;
-    const long long qi = blockIdx.x;
-    if (qi >= a.nq) return;
+    if ((long long)blockIdx.x >= a.nq) return;
+    const long long qi = list_index(a, blockIdx.x);
     const int2 pq = a.quartets[qi];
     const PairInfo P = a.pairs[pq.x];
     const PairInfo Q = a.pairs[pq.y];

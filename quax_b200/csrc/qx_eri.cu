@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <functional>
 #include <memory>
@@ -199,6 +200,7 @@ struct ClassWork {
     long long nq = 0;
     int2* d_q = nullptr;       // this rank's quartets: a view into d_q_full
     int2* d_q_full = nullptr;  // the class's full screened list (owned)
+    int* d_order = nullptr;    // processing order of this rank's quartets (into qx_handle::d_orders; null: list order)
     long long nq_full = 0;
     long long unique_base = 0;
     long long prims = 0;       // primitive quartets of the class
@@ -244,8 +246,10 @@ struct qx_handle {
     // all shell pairs s1 >= s2 (reference order), canonical records
     std::vector<PairInfo> pairs;
     std::vector<int> pcls;
+    std::vector<int> nfull;  // primitive pairs per pair before the negligible ones were dropped (the lists' sort key)
     PrimPair* d_prims = nullptr;
     PairInfo* d_pairs = nullptr;
+    int* d_orders = nullptr;  // the classes' processing orders
     double* d_boys = nullptr;
     const double* d_rys = nullptr;  // Rys node/weight table (module data, not owned)
     int* d_err = nullptr;
@@ -292,6 +296,59 @@ static void host_parallel(int nt, F&& f) {
     for (int t = 1; t < nt; ++t) pool.emplace_back([&f, t] { f(t); });
     f(0);
     for (auto& th : pool) th.join();
+}
+
+// Processing order of the classes' views (lists[c] on the host): by primitive quartets,
+// largest first, stable.  The list itself keeps the order of the contracted primitive
+// counts (the unique layout); once negligible primitive pairs are dropped, neighbours
+// there differ several-fold in work, and a straight-line kernel's warp takes as long as
+// its longest lane.  A class of equal counts needs none.
+static int build_orders(qx_handle* h, const int2* const* lists) {
+    cudaFree(h->d_orders);
+    h->d_orders = nullptr;
+    constexpr int NB = 4096;
+    long long total = 0;
+    std::vector<long long> off(QX_NCLS_ALL, 0);
+    for (int c = 0; c < QX_NCLS_ALL; ++c) {
+        h->work[c].d_order = nullptr;
+        off[c] = total;
+        total += h->work[c].nq;
+    }
+    std::unique_ptr<int[]> order(new int[(size_t)std::max(1LL, total)]);
+    std::vector<char> uniform(QX_NCLS_ALL, 1);
+    std::atomic<int> next{0};
+    const int nt = total < 65536 ? 1 : (int)std::min(8u, std::max(1u, std::thread::hardware_concurrency()));
+    host_parallel(nt, [&](int) {
+        std::vector<int> pos(NB + 1);
+        std::vector<unsigned short> key;
+        for (int i; (i = next.fetch_add(1)) < QX_NCLS_ALL;) {
+            const int c = h->order[i];
+            const long long nq = h->work[c].nq;
+            if (!nq) continue;
+            const int2* L = lists[c];
+            std::fill(pos.begin(), pos.end(), 0);
+            key.resize((size_t)nq);
+            for (long long q = 0; q < nq; ++q) {
+                key[q] = (unsigned short)(NB - std::min(h->pairs[L[q].x].nprim * h->pairs[L[q].y].nprim, NB));
+                ++pos[key[q] + 1];
+                if (key[q] != key[0]) uniform[c] = 0;
+            }
+            if (uniform[c]) continue;
+            for (int k = 0; k < NB; ++k) pos[k + 1] += pos[k];
+            int* o = order.get() + off[c];
+            for (long long q = 0; q < nq; ++q) o[pos[key[q]]++] = (int)q;
+        }
+    });
+    if (std::all_of(uniform.begin(), uniform.end(), [](char u) { return u != 0; })) return QX_OK;
+    if (cudaMalloc((void**)&h->d_orders, sizeof(int) * total) != cudaSuccess) {
+        cudaGetLastError();
+        h->d_orders = nullptr;
+        return fail(QX_E_NOMEM, "processing order of %lld quartets", total);
+    }
+    QX_CUDA(cudaMemcpy(h->d_orders, order.get(), sizeof(int) * total, cudaMemcpyHostToDevice));
+    for (int c = 0; c < QX_NCLS_ALL; ++c)
+        if (!uniform[c]) h->work[c].d_order = h->d_orders + off[c];
+    return QX_OK;
 }
 
 static int ensure_split_tasks(qx_handle* h, int c, bool need_dacc = false, const int2* list = nullptr,
@@ -417,6 +474,7 @@ static int pair_index(int s1, int s2) { return s1 * (s1 + 1) / 2 + s2; }  // s1 
 static void free_handle(qx_handle* h) {
     if (!h) return;
     cudaFree(h->d_prims);
+    cudaFree(h->d_orders);
     cudaFree(h->d_pairs);
     cudaFree(h->d_boys);
     cudaFree(h->d_err);
@@ -458,7 +516,10 @@ static int run_class(qx_handle* h, int cls, int mode, const int2* d_q, long long
     a.dens = dens;
     a.log2g = eng == ENG_SL ? log2g : 0;
     a.err = h->d_err;
-    if (d_q == h->work[cls].d_q) a.nq64 = h->work[cls].nq64;
+    if (d_q == h->work[cls].d_q) {
+        a.nq64 = h->work[cls].nq64;
+        a.order = h->work[cls].d_order;
+    }
     if (mode == MODE_JK && h->jk_thr > 0.0) {
         a.jk_thr = h->jk_thr;
         a.jk_kpair = h->d_kpair;
@@ -570,7 +631,7 @@ extern "C" int qx_initialize(int natom, const double* coords, int nshell, const 
     trace.mark("shells");
     // pair records
     std::vector<PrimPair> prims;
-    build_pairs(shells, coords, prims, h->pairs, h->pcls);
+    build_pairs(shells, coords, ints_tol, prims, h->pairs, h->pcls, &h->nfull);
     const std::vector<double>& boys = boys_table();
     const int np = (int)h->pairs.size();
     {
@@ -678,7 +739,7 @@ extern "C" int qx_initialize(int natom, const double* coords, int nshell, const 
     cut_i[0] = 0;
     for (int t = 1; t < nt; ++t) cut_i[t] = (size_t)(nk * std::sqrt((double)t / nt));
     auto key = [&](int pb, int pk) {
-        return NKEY - 1 - std::min((h->pairs[pb].nprim - 1) * 64 + (h->pairs[pk].nprim - 1), NKEY - 1);
+        return NKEY - 1 - std::min((h->nfull[pb] - 1) * 64 + (h->nfull[pk] - 1), NKEY - 1);
     };
     auto visit = [&](int t, auto&& fn) {
         for (size_t i = cut_i[t]; i < cut_i[t + 1]; ++i)
@@ -745,7 +806,6 @@ extern "C" int qx_initialize(int natom, const double* coords, int nshell, const 
             }
             if (g_class_scratch[c] && h->plain_eng[c] == ENG_SL)
                 QX_ALLOC(w.scratch, sizeof(double) * g_class_scratch[c] * launch_threads(w.nq, w.log2g));
-            sorted[c].reset();
         }
     }
     h->unique_size = base;
@@ -753,6 +813,16 @@ extern "C" int qx_initialize(int natom, const double* coords, int nshell, const 
     for (int c = 0; c < QX_NCLS_ALL; ++c) h->order[c] = c;
     std::sort(h->order, h->order + QX_NCLS_ALL,
               [&](int x, int y) { return h->work[x].prims * g_class_nout[x] > h->work[y].prims * g_class_nout[y]; });
+    {
+        const int2* lists[QX_NCLS_ALL];
+        for (int c = 0; c < QX_NCLS_ALL; ++c) lists[c] = sorted[c].get();
+        const int rc = build_orders(h, lists);
+        if (rc) {
+            free_handle(h);
+            return rc;
+        }
+    }
+    trace.mark("processing orders");
     for (int i = 0; i < QX_NSTREAMS; ++i) {
         if (cudaStreamCreateWithFlags(&h->streams[i], cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&h->done[i], cudaEventDisableTiming) != cudaSuccess) {
@@ -807,6 +877,8 @@ extern "C" int qx_partition_costs(const double* cost, long long n, int nranks, l
 static int rebuild_views(qx_handle* h) {
     QX_CUDA(cudaDeviceSynchronize());
     const int rank = h->shard_rank, nranks = h->shard_n;
+    std::vector<std::vector<int2>> full(QX_NCLS_ALL);
+    const int2* lists[QX_NCLS_ALL];
     long long base = 0;
     h->nunique = 0;
     for (int c = 0; c < QX_NCLS_ALL; ++c) {
@@ -821,8 +893,9 @@ static int rebuild_views(qx_handle* h) {
         w.slice_t.clear();
         long long lo = 0, hi = w.nq_full;
         long long prims = 0;
+        std::vector<int2>& L = full[c];
+        L.resize((size_t)w.nq_full);
         if (w.nq_full) {
-            std::vector<int2> L((size_t)w.nq_full);
             QX_CUDA(cudaMemcpy(L.data(), w.d_q_full, sizeof(int2) * w.nq_full, cudaMemcpyDeviceToHost));
             std::vector<double> cost((size_t)w.nq_full);
             for (long long i = 0; i < w.nq_full; ++i)
@@ -841,8 +914,12 @@ static int rebuild_views(qx_handle* h) {
         w.unique_base = base;
         base += w.nq * g_class_nout[c];
         h->nunique += w.nq;
+        lists[c] = L.data() + lo;
     }
     h->unique_size = base;
+    int rc = build_orders(h, lists);
+    if (rc) return rc;
+    QX_CUDA(cudaDeviceSynchronize());  // the order lists have landed before any stream reads them
     return QX_OK;
 }
 
@@ -880,7 +957,7 @@ extern "C" int qx_set_precision(qx_handle* h, double bound) {
         QX_CUDA(cudaMemcpy(L.data(), w.d_q_full, sizeof(int2) * w.nq_full, cudaMemcpyDeviceToHost));
         // restore the set-up order (bra nprim, then ket nprim, largest first), then
         // split by the bound
-        auto key = [&](const int2& q) { return h->pairs[q.x].nprim * 64 + h->pairs[q.y].nprim; };
+        auto key = [&](const int2& q) { return h->nfull[q.x] * 64 + h->nfull[q.y]; };
         std::stable_sort(L.begin(), L.end(), [&](const int2& x, const int2& y) { return key(x) > key(y); });
         // FP32 recurrence errors are amplified by the HRR's cancellations, about
         // tenfold per transfer step (measured relative error of the FP32 path:
@@ -1047,6 +1124,7 @@ static EriArgs class_args(qx_handle* h, int c, double* out) {
     a.out2 = nullptr;
     a.dens = nullptr;
     a.nq64 = w.nq64;
+    a.order = w.d_order;
     return a;
 }
 
@@ -1133,6 +1211,7 @@ static int run_deriv_class(qx_handle* h, int c, int mode, double* out, const dou
         for (size_t sl = 0; sl + 1 < w.slice_q.size(); ++sl) {
             EriArgs a = class_args(h, c, out);
             a.quartets = w.d_q + w.slice_q[sl];
+            if (w.slice_q.size() > 2) a.order = nullptr;  // the order is the whole list's
             a.nq = w.slice_q[sl + 1] - w.slice_q[sl];
             a.nq64 = w.nq64 - w.slice_q[sl];
             const int2* tk = w.d_dtasks + w.slice_t[sl];
@@ -1783,6 +1862,7 @@ extern "C" int qx_deriv_tile(qx_handle* h, int cls, long long q0, long long q1, 
     EriArgs a = class_args(h, cls, B);
     a.quartets = w.d_q + q0;
     a.nq = q1 - q0;
+    a.order = nullptr;
     a.nq64 = w.nq64 >= q1 ? a.nq : std::max(0LL, w.nq64 - q0);
     if (h->deriv_eng[cls] == ENG_WARP) {
         WarpArgs wa;

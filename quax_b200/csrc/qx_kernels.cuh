@@ -28,6 +28,9 @@ struct EriArgs {
     // mixed precision: quartets [nq64, nq) of the list run their recurrences in
     // FP32 (warp and split engines); the default keeps every quartet FP64
     long long nq64 = 0x7fffffffffffffffLL;
+    // processing order: the i-th quartet a kernel takes is quartets[order[i]] (null: the
+    // list order).  Positions in the unique layout stay those of the list.
+    const int* order = nullptr;
     // density screening of J/K (MODE_JK): a quartet is skipped when
     // sqrt(K_ab) sqrt(K_cd) max(|D| over its six shell-pair blocks) < jk_thr
     const double* jk_kpair = nullptr;  // sqrt(Schwarz K) per pair record
@@ -41,6 +44,10 @@ struct EriArgs {
     // timeout through the error word
     int wait_limit = 1 << 22;
 };
+
+__device__ __forceinline__ long long list_index(const EriArgs& a, long long i) {
+    return a.order ? __ldg(a.order + i) : i;
+}
 
 // True when density screening drops this quartet from J/K.
 __device__ __forceinline__ bool jk_screened(const EriArgs& a, int2 pq, const PairInfo& P, const PairInfo& Q) {
@@ -212,9 +219,10 @@ __global__ void __launch_bounds__(AccPolicy<EriCls<LA, LB, LC, LD>::NACC>::bs) k
     using C = EriCls<LA, LB, LC, LD>;
     using Pol = AccPolicy<C::NACC>;
     const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long qi = gt >> a.log2g;
+    long long qi = gt >> a.log2g;
     const int sub = (int)(gt & ((1 << a.log2g) - 1));
     bool active = qi < a.nq;
+    if (active) qi = list_index(a, qi);
     // every lane stays to the end: the group reduction shuffles over the full warp
     const int2 pq = active ? a.quartets[qi] : make_int2(0, 0);
     const PairInfo P = a.pairs[pq.x];

@@ -159,7 +159,7 @@ extern "C" int qx_compute_2e_int_noalloc(int natom, const double* coords, int ns
     std::vector<PrimPair> prims;
     std::vector<PairInfo> pairs;
     std::vector<int> pcls;
-    build_pairs(shells, coords, prims, pairs, pcls);
+    build_pairs(shells, coords, ints_tol, prims, pairs, pcls);
     const int np = (int)pairs.size();
     // --- scratch layout part 1: Boys | prims | pairs | K per pair | diagonal lists ---
     const size_t o_prims = align256(kBoysBytes);

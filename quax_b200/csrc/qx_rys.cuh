@@ -861,6 +861,7 @@ __global__ void __launch_bounds__(RysCls<LA, LB, LC, LD, KIND>::BS, RysCls<LA, L
             qi = w / ra.nchunk;
             ch = (int)(w - qi * ra.nchunk);
         }
+        qi = list_index(a, qi);
         const int2 pq = a.quartets[qi];
         const PairInfo P = a.pairs[pq.x];
         const PairInfo Q = a.pairs[pq.y];

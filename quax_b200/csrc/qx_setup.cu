@@ -1,8 +1,11 @@
 // qx_setup.cu -- host-side set-up shared by qx_initialize and the no-alloc path.
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <mutex>
+#include <utility>
+#include <vector>
 
 #include "quax_b200.h"
 #include "qx_setup.h"
@@ -71,13 +74,16 @@ int normalize_shells(const char* who, int natom, int nshell, const int* shell_l,
     return QX_OK;
 }
 
-void build_pairs(const ShellTables& t, const double* coords, std::vector<PrimPair>& prims,
-                 std::vector<PairInfo>& pairs, std::vector<int>& pcls) {
+void build_pairs(const ShellTables& t, const double* coords, double tol, std::vector<PrimPair>& prims,
+                 std::vector<PairInfo>& pairs, std::vector<int>& pcls, std::vector<int>* nfull) {
     const int nshell = (int)t.l.size();
     const double kfac = std::sqrt(2.0) * std::pow(M_PI, 1.25);
     prims.clear();
     pairs.clear();
     pcls.clear();
+    if (nfull) nfull->clear();
+    const double cut = 1e-18 * std::min(tol, 1e-10);
+    std::vector<std::pair<PrimPair, double>> cand;  // record and size bound
     for (int s1 = 0; s1 < nshell; ++s1)
         for (int s2 = 0; s2 <= s1; ++s2) {
             int f = s1, g = s2;
@@ -89,11 +95,13 @@ void build_pairs(const ShellTables& t, const double* coords, std::vector<PrimPai
             pi.ABx = A[0] - B[0]; pi.ABy = A[1] - B[1]; pi.ABz = A[2] - B[2];
             const double AB2 = pi.ABx * pi.ABx + pi.ABy * pi.ABy + pi.ABz * pi.ABz;
             pi.prim_off = (int)prims.size();
-            pi.nprim = t.nprim[f] * t.nprim[g];
             pi.bf1 = t.bf[f]; pi.bf2 = t.bf[g];
             pi.s1 = f; pi.s2 = g;
             pi.atom1 = t.atom[f]; pi.atom2 = t.atom[g];
             pi.l1 = t.l[f]; pi.l2 = t.l[g];
+            const double AB = std::sqrt(AB2);
+            double best = -1.0;
+            cand.clear();
             for (int p = 0; p < t.nprim[f]; ++p)
                 for (int q = 0; q < t.nprim[g]; ++q) {
                     const double a = t.alpha[t.poff[f] + p], b = t.alpha[t.poff[g] + q];
@@ -111,8 +119,25 @@ void build_pairs(const ShellTables& t, const double* coords, std::vector<PrimPai
                     r.Px = A[0] + r.PAx; r.Py = A[1] + r.PAy; r.Pz = A[2] + r.PAz;
                     r.K = kfac * ca * cb * std::exp(-a * b / r.zeta * AB2) / r.zeta;
                     r.alpha = a;
-                    prims.push_back(r);
+                    // charge of the primitive pair's density: c_a c_b exp(-mu AB^2)
+                    // (pi / zeta)^{3/2} times the extent of its polynomials, and times
+                    // the (2 zeta)^{1/4} of a Coulomb norm
+                    const double w = 1.0 / std::sqrt(r.zeta);
+                    const double size = std::fabs(r.K) * std::pow(r.zeta, -0.25) * std::pow(b / r.zeta * AB + w, pi.l1) *
+                                        std::pow(a / r.zeta * AB + w, pi.l2);
+                    best = std::max(best, size);
+                    // every nuclear derivative adds at most a factor of about
+                    // 2 mu AB + 2 sqrt(zeta) < 8 sqrt(zeta) down to exp(-16); beyond, the
+                    // two decades of room cover it
+                    cand.push_back({r, size * (1.0 + 64.0 * r.zeta) * (1.0 + 64.0 * r.zeta)});
                 }
+            // both below the absolute cut and negligible in the pair itself, so that the
+            // Schwarz values keep their relative accuracy; the largest one always stays
+            const double drop = std::min(cut, 1e-18 * best);
+            for (const auto& c : cand)
+                if (!(c.second < drop)) prims.push_back(c.first);
+            pi.nprim = (int)prims.size() - pi.prim_off;
+            if (nfull) nfull->push_back(t.nprim[f] * t.nprim[g]);
             pairs.push_back(pi);
             pcls.push_back(pi.l1 * (pi.l1 + 1) / 2 + pi.l2);
         }

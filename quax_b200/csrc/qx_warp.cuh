@@ -259,8 +259,9 @@ __global__ void __launch_bounds__(WARP_QPB * 32) k_warp(WarpArgs wa, int mode) {
     // wpq = 4: the block's four warps split one quartet's primitive batches
     const int wpq = wa.wpq;
     const int sub = warp % wpq;
-    const long long qi = (long long)blockIdx.x * (WARP_QPB / wpq) + warp / wpq;
-    if (qi >= a.nq) return;  // whole warp (whole block when wpq = 4)
+    const long long ti = (long long)blockIdx.x * (WARP_QPB / wpq) + warp / wpq;
+    if (ti >= a.nq) return;  // whole warp (whole block when wpq = 4)
+    const long long qi = list_index(a, ti);
     extern __shared__ double warp_sm[];
     double* H = warp_sm + (size_t)warp * W::SMEM_PER_WARP;  // accumulators = HRR leaves
     double* geo = H + W::HSLOTS;                             // 6 geometry factors + constants -8..7
