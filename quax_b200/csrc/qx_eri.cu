@@ -250,6 +250,10 @@ struct qx_handle {
     PrimPair* d_prims = nullptr;
     PairInfo* d_pairs = nullptr;
     int* d_orders = nullptr;  // the classes' processing orders
+    // pair records and primitive pairs with none dropped, for the second-derivative
+    // programs of the s and p classes (null: nothing was dropped from their pairs)
+    PairInfo* d_pairs_all = nullptr;
+    PrimPair* d_prims_all = nullptr;
     double* d_boys = nullptr;
     const double* d_rys = nullptr;  // Rys node/weight table (module data, not owned)
     int* d_err = nullptr;
@@ -267,6 +271,7 @@ struct qx_handle {
     int deriv_eng[QX_NCLS_ALL];
     int wpq[QX_NCLS_ALL];        // warps per quartet, plain warp kernels
     int wpq_deriv[QX_NCLS_ALL];  // warps per quartet, derivative warp kernels
+    int wpq_deriv2[QX_NCLS_ALL]; // second-derivative warp kernels (they run every primitive)
     int rys_lp[QX_NCLS_ALL];     // Rys adjoint gradient: 1 = level-parallel table build (RK_GRADL)
     int shard_rank = 0, shard_n = 1;
     int prim_stage = 0;  // split-mode VRR: primitive pairs staged per warp (2 x largest pair), 0 = off
@@ -475,6 +480,8 @@ static void free_handle(qx_handle* h) {
     if (!h) return;
     cudaFree(h->d_prims);
     cudaFree(h->d_orders);
+    cudaFree(h->d_pairs_all);
+    cudaFree(h->d_prims_all);
     cudaFree(h->d_pairs);
     cudaFree(h->d_boys);
     cudaFree(h->d_err);
@@ -600,7 +607,7 @@ extern "C" int qx_initialize(int natom, const double* coords, int nshell, const 
     cudaGetDevice(&h->device);
     choose_engines(h);
     for (int c = 0; c < QX_NCLS_ALL; ++c) {
-        h->wpq[c] = h->wpq_deriv[c] = 1;
+        h->wpq[c] = h->wpq_deriv[c] = h->wpq_deriv2[c] = 1;
         h->rys_lp[c] = 0;
     }
     h->natom = natom;
@@ -631,7 +638,9 @@ extern "C" int qx_initialize(int natom, const double* coords, int nshell, const 
     trace.mark("shells");
     // pair records
     std::vector<PrimPair> prims;
-    build_pairs(shells, coords, ints_tol, prims, h->pairs, h->pcls, &h->nfull);
+    std::vector<PrimPair> prims_all;
+    std::vector<int> all_off;
+    build_pairs(shells, coords, ints_tol, prims, h->pairs, h->pcls, &h->nfull, &prims_all, &all_off);
     const std::vector<double>& boys = boys_table();
     const int np = (int)h->pairs.size();
     {
@@ -664,6 +673,20 @@ extern "C" int qx_initialize(int natom, const double* coords, int nshell, const 
     cudaMemcpy(h->d_pairs, h->pairs.data(), sizeof(PairInfo) * np, cudaMemcpyHostToDevice);
     cudaMemcpy(h->d_boys, boys.data(), sizeof(double) * boys.size(), cudaMemcpyHostToDevice);
     cudaMemset(h->d_err, 0, sizeof(int));
+    bool dropped = false;
+    for (int p = 0; p < np; ++p) dropped = dropped || (h->pairs[p].l1 <= 1 && h->pairs[p].nprim < h->nfull[p]);
+    if (dropped) {
+        std::vector<PairInfo> all(h->pairs);
+        for (int p = 0; p < np; ++p)
+            if (all[p].l1 <= 1) {
+                all[p].prim_off = all_off[p];
+                all[p].nprim = h->nfull[p];
+            }
+        QX_ALLOC(h->d_prims_all, sizeof(PrimPair) * prims_all.size());
+        QX_ALLOC(h->d_pairs_all, sizeof(PairInfo) * np);
+        cudaMemcpy(h->d_prims_all, prims_all.data(), sizeof(PrimPair) * prims_all.size(), cudaMemcpyHostToDevice);
+        cudaMemcpy(h->d_pairs_all, all.data(), sizeof(PairInfo) * np, cudaMemcpyHostToDevice);
+    }
     // global accumulator scratch, sized for the largest launch that needs it
     {
         long long need = 0;
@@ -751,16 +774,18 @@ extern "C" int qx_initialize(int natom, const double* coords, int nshell, const 
             }
     };
     std::vector<long long> cnt((size_t)nt * QX_NCLS_ALL * NKEY, 0);
-    std::vector<long long> tprims((size_t)nt * QX_NCLS_ALL, 0);
+    std::vector<long long> tprims((size_t)nt * QX_NCLS_ALL, 0), tfull((size_t)nt * QX_NCLS_ALL, 0);
     host_parallel(nt, [&](int t) {
         long long* C = cnt.data() + (size_t)t * QX_NCLS_ALL * NKEY;
         long long* P = tprims.data() + (size_t)t * QX_NCLS_ALL;
+        long long* F = tfull.data() + (size_t)t * QX_NCLS_ALL;
         visit(t, [&](int c, int k, int pb, int pk) {
             C[(size_t)c * NKEY + k]++;
             P[c] += (long long)h->pairs[pb].nprim * h->pairs[pk].nprim;
+            F[c] += (long long)h->nfull[pb] * h->nfull[pk];
         });
     });
-    std::vector<long long> nq_c(QX_NCLS_ALL, 0), prims_c(QX_NCLS_ALL, 0);
+    std::vector<long long> nq_c(QX_NCLS_ALL, 0), prims_c(QX_NCLS_ALL, 0), full_c(QX_NCLS_ALL, 0);
     for (int c = 0; c < QX_NCLS_ALL; ++c) {
         long long run = 0;
         for (int k = 0; k < NKEY; ++k)
@@ -771,7 +796,10 @@ extern "C" int qx_initialize(int natom, const double* coords, int nshell, const 
                 run += v;
             }
         nq_c[c] = run;
-        for (int t = 0; t < nt; ++t) prims_c[c] += tprims[(size_t)t * QX_NCLS_ALL + c];
+        for (int t = 0; t < nt; ++t) {
+            prims_c[c] += tprims[(size_t)t * QX_NCLS_ALL + c];
+            full_c[c] += tfull[(size_t)t * QX_NCLS_ALL + c];
+        }
     }
     std::vector<std::unique_ptr<int2[]>> sorted(QX_NCLS_ALL);
     for (int c = 0; c < QX_NCLS_ALL; ++c)
@@ -789,6 +817,7 @@ extern "C" int qx_initialize(int natom, const double* coords, int nshell, const 
         w.prims = prims_c[c];
         w.log2g = h->plain_eng[c] == ENG_SL ? choose_log2g(w.nq, w.prims) : 0;
         h->wpq[c] = h->wpq_deriv[c] = choose_wpq(w.nq, w.prims);
+        h->wpq_deriv2[c] = choose_wpq(w.nq, full_c[c]);
         w.unique_base = base;
         base += w.nq * g_class_nout[c];
         h->nunique += w.nq;
@@ -1295,7 +1324,11 @@ static int run_all_deriv2(qx_handle* h, int mode, double* out, int slice, cudaSt
         }
         WarpArgs wa;
         wa.e = class_args(h, c, out);
-        wa.wpq = h->wpq_deriv[c];
+        if (h->d_pairs_all) {
+            wa.e.pairs = h->d_pairs_all;
+            wa.e.prims = h->d_prims_all;
+        }
+        wa.wpq = h->wpq_deriv2[c];
         wa.D = D;
         wa.cj = cj;
         wa.ck = ck;

@@ -75,7 +75,8 @@ int normalize_shells(const char* who, int natom, int nshell, const int* shell_l,
 }
 
 void build_pairs(const ShellTables& t, const double* coords, double tol, std::vector<PrimPair>& prims,
-                 std::vector<PairInfo>& pairs, std::vector<int>& pcls, std::vector<int>* nfull) {
+                 std::vector<PairInfo>& pairs, std::vector<int>& pcls, std::vector<int>* nfull,
+                 std::vector<PrimPair>* all, std::vector<int>* all_off) {
     const int nshell = (int)t.l.size();
     const double kfac = std::sqrt(2.0) * std::pow(M_PI, 1.25);
     prims.clear();
@@ -137,6 +138,11 @@ void build_pairs(const ShellTables& t, const double* coords, double tol, std::ve
             for (const auto& c : cand)
                 if (!(c.second < drop)) prims.push_back(c.first);
             pi.nprim = (int)prims.size() - pi.prim_off;
+            if (all) {
+                all_off->push_back((int)all->size());
+                if (pi.l1 <= 1)
+                    for (const auto& c : cand) all->push_back(c.first);
+            }
             if (nfull) nfull->push_back(t.nprim[f] * t.nprim[g]);
             pairs.push_back(pi);
             pcls.push_back(pi.l1 * (pi.l1 + 1) / 2 + pi.l2);

@@ -37,8 +37,13 @@ int normalize_shells(const char* who, int natom, int nshell, const int* shell_l,
 // of its integrals.  On the synthetic workloads (exponents 0.08 to 5e3, atoms 2 to 20
 // bohr apart) half of the primitive pairs, and three quarters of the primitive quartets,
 // carry an exp(-mu R^2) below that.
+//
+// all (if not null) receives every primitive pair of the s and p pairs, in order, and
+// all_off its range per pair: the second-derivative programs of those classes sum
+// weights of (2 alpha)^2 that cancel, and any other grouping of that sum is visible.
 void build_pairs(const ShellTables& t, const double* coords, double tol, std::vector<PrimPair>& prims,
-                 std::vector<PairInfo>& pairs, std::vector<int>& pcls, std::vector<int>* nfull = nullptr);
+                 std::vector<PairInfo>& pairs, std::vector<int>& pcls, std::vector<int>* nfull = nullptr,
+                 std::vector<PrimPair>* all = nullptr, std::vector<int>* all_off = nullptr);
 
 // Boys table F_m(T_g) (BOYS_NG x BOYS_NM, row-major [g][m]); built once per
 // process on first use.
