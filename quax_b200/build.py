@@ -79,8 +79,8 @@ def _compile(src: str, verbose: bool):
     if os.path.exists(obj) and os.path.getmtime(obj) >= _deps_mtime(src):
         return obj, False
     flags = NVCC_FLAGS
-    if os.path.basename(src).startswith("k_rys_"):
-        # the 55 Rys-engine units carry ~7 kernels each; their line tables would
+    if os.path.basename(src).startswith(("k_rys_", "k_tile_")):
+        # the Rys and tile units carry several kernels per class; their line tables would
         # more than double the library, so they are built without -lineinfo
         flags = [f for f in NVCC_FLAGS if f != "-lineinfo"]
     cmd = [nvcc()] + flags + ["-c", src, "-o", obj]

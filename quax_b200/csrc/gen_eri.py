@@ -1111,17 +1111,15 @@ class _Out:
 
 # Highest shell angular momentum of the Rys engine (every class up to (ff|ff)).
 RYS_LMAX = 3
-RYS_ALL_KINDS = ("RK_PLAIN", "RK_GRAD", "RK_GRADL", "RK_HVP", "RK_GRADT", "RK_DER1", "RK_DER2", "RK_DER3",
-                 "RK_DER4")
+RYS_ALL_KINDS = ("RK_HVP", "RK_GRADT", "RK_DER1", "RK_DER2", "RK_DER3", "RK_DER4")
 
 
 def gen_rys(here, lmax_os):
     """One translation unit per class up to RYS_LMAX with the Rys launcher
-    qx_launch_rys_<id>(args, kind, mode, nwork, stream) -> 0, or 1 when the kind
-    does not fit shared memory for the class.  Every class gets every kind: for
-    the f classes this is the only engine, for the l <= lmax_os classes it
-    serves the second- and higher-order derivatives and is an autotuner
-    candidate next to the Obara-Saika programs."""
+    qx_launch_rys_<id>(args, kind, nwork, stream) -> 0, or 1 when the kind does
+    not fit shared memory for the class.  Every class gets every kind: derivative
+    tensors, tiles and Hessian-vector products of the f classes, and for the
+    l <= lmax_os classes the derivatives of second and higher order."""
     del lmax_os
     qc = quartet_classes(RYS_LMAX)
     for i, (a, b, c, d) in enumerate(qc):
@@ -1129,10 +1127,10 @@ def gen_rys(here, lmax_os):
         L = ["// Generated by quax_b200/csrc/gen_eri.py -- do not edit by hand.",
              f"// Rys-engine launchers of class ({a}{b}|{c}{d}).",
              '#include "../qx_rys.cuh"',
-             f"int qx_launch_rys_{i:02d}(const qx::RysArgs& ra, int kind, int mode, long long nwork, cudaStream_t s) {{",
+             f"int qx_launch_rys_{i:02d}(const qx::RysArgs& ra, int kind, long long nwork, cudaStream_t s) {{",
              "    switch (kind) {"]
         for k in kinds:
-            L.append(f"    case qx::{k}: return qx::launch_rys<{a}, {b}, {c}, {d}, qx::{k}>(ra, mode, nwork, s) ? 0 : 1;")
+            L.append(f"    case qx::{k}: return qx::launch_rys<{a}, {b}, {c}, {d}, qx::{k}>(ra, nwork, s) ? 0 : 1;")
         L += ["    default: return 1;", "    }", "}"]
         with _Out(os.path.join(here, "gen", f"k_rys_{i:02d}.cu")) as f:
             f.write("\n".join(L) + "\n")
@@ -1144,6 +1142,24 @@ def gen_rys(here, lmax_os):
          "#define QX_FOR_EACH_CLASS_ALL(X) " + " ".join(f"X({i:02d}, {a}, {b}, {c}, {d})" for i, (a, b, c, d) in enumerate(qc))]
     with _Out(os.path.join(here, "gen", "rys_index.cuh")) as f:
         f.write("\n".join(H) + "\n")
+
+
+def gen_tile(here):
+    """One translation unit per class up to RYS_LMAX with the tile engine's launcher
+    qx_launch_tile_<id>(args, kind, mode, nquartets, largest primitive count, stream)."""
+    qc = quartet_classes(RYS_LMAX)
+    for i, (a, b, c, d) in enumerate(qc):
+        L = ["// Generated by quax_b200/csrc/gen_eri.py -- do not edit by hand.",
+             f"// Tile-engine launchers of class ({a}{b}|{c}{d}).",
+             '#include "../qx_tile.cuh"',
+             f"void qx_launch_tile_{i:02d}(qx::TileArgs& ta, int kind, int mode, long long nq, int max_prims, "
+             "cudaStream_t s) {"]
+        for k in ("TK_PLAIN", "TK_GRAD"):
+            L.append(f"    if (kind == qx::{k}) return qx::launch_tile<qx::TileCls<{a}, {b}, {c}, {d}, qx::{k}>>"
+                     "(ta, mode, nq, max_prims, s);")
+        L += ["}"]
+        with _Out(os.path.join(here, "gen", f"k_tile_{i:02d}.cu")) as f:
+            f.write("\n".join(L) + "\n")
 
 
 def main():
@@ -1224,6 +1240,7 @@ def main():
     with _Out(os.path.join(here, "gen", "der_tables.cuh")) as f:
         f.write(gen_coop_deriv(list(enumerate(qc))))
     gen_rys(here, lmax)
+    gen_tile(here)
 
 
 if __name__ == "__main__":

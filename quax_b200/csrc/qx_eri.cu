@@ -32,6 +32,7 @@
 #include "quax_b200.h"
 #include "qx_warp.cuh"
 #include "qx_rys.cuh"
+#include "qx_tile.cuh"
 #include "qx_setup.h"
 #include "gen/warp_index.cuh"
 #include "gen/rys_index.cuh"
@@ -96,11 +97,17 @@ static const int g_class_l[QX_NCLS_ALL][4] = {
 };
 // Rys-engine launchers, one per class (gen/k_rys_<id>.cu): 0 = launched, 1 = this
 // kind is not compiled for the class or its tables exceed shared memory.
-typedef int (*RysLaunch)(const qx::RysArgs&, int kind, int mode, long long nwork, cudaStream_t);
-#define QX_DECL_RYS(id, a, b, c, d) int qx_launch_rys_##id(const qx::RysArgs&, int, int, long long, cudaStream_t);
+typedef int (*RysLaunch)(const qx::RysArgs&, int kind, long long nwork, cudaStream_t);
+#define QX_DECL_RYS(id, a, b, c, d) int qx_launch_rys_##id(const qx::RysArgs&, int, long long, cudaStream_t);
 QX_FOR_EACH_CLASS_ALL(QX_DECL_RYS)
 #undef QX_DECL_RYS
 static RysLaunch g_rys_launch[QX_NCLS_ALL];
+// Tile-engine launchers, one per class (gen/k_tile_<id>.cu).
+typedef void (*TileLaunch)(qx::TileArgs&, int kind, int mode, long long nq, int max_prims, cudaStream_t);
+#define QX_DECL_TILE(id, a, b, c, d) void qx_launch_tile_##id(qx::TileArgs&, int, int, long long, int, cudaStream_t);
+QX_FOR_EACH_CLASS_ALL(QX_DECL_TILE)
+#undef QX_DECL_TILE
+static TileLaunch g_tile_launch[QX_NCLS_ALL];
 const double* qx_rys_table();
 static int g_coop_idx[QX_NCLS_ALL];
 static int g_der_idx[QX_NCLS_ALL];
@@ -139,8 +146,9 @@ QX_FOR_EACH_DSPLIT(QX_DECL_DS)
 // cooperative HRR; ENG_WSPLIT (plain): the same VRR split + the warp HRR.
 // ENG_DSPLIT (derivatives): the split VRR into item-order accumulators + the warp
 // kernel's own HRR and epilogue.
-// ENG_RYS (plain and derivatives): the Rys-quadrature engine (qx_rys.cuh), the only
-// engine of the classes with an f shell.
+// ENG_RYS: Rys quadrature -- the tile kernels (qx_tile.cuh) for plain integrals and the
+// adjoint gradient, qx_rys.cuh for derivative tensors and tiles; the only engine of the
+// classes with an f shell.
 enum { ENG_SL = 0, ENG_WARP = 1, ENG_COOP = 2, ENG_WVRR = 3, ENG_WSPLIT = 4, ENG_DSPLIT = 5, ENG_RYS = 6 };
 int qx_der_index(int cls);
 void qx_launch_der_split(int der_idx, const qx::EriArgs& a, int mode, const double* D, double cj, double ck,
@@ -187,6 +195,9 @@ static bool init_class_tables() {
 #define QX_RYS_ENTRY(id, a, b, c, d) g_rys_launch[1##id - 100] = &qx_launch_rys_##id;
     QX_FOR_EACH_CLASS_ALL(QX_RYS_ENTRY)
 #undef QX_RYS_ENTRY
+#define QX_TILE_ENTRY(id, a, b, c, d) g_tile_launch[1##id - 100] = &qx_launch_tile_##id;
+    QX_FOR_EACH_CLASS_ALL(QX_TILE_ENTRY)
+#undef QX_TILE_ENTRY
 #define QX_SL_ENTRY(id, a, b, c, d)                            \
     g_eri_launch[id] = &qx_launch_eri_##id;                    \
     g_class_scratch[id] = qx::scratch_per_quartet<a, b, c, d>();
@@ -204,6 +215,7 @@ struct ClassWork {
     long long nq_full = 0;
     long long unique_base = 0;
     long long prims = 0;       // primitive quartets of the class
+    int max_prims = 0;         // of its largest quartet
     int log2g = 0;             // lanes per quartet = 2^log2g
     double* scratch = nullptr; // global accumulators (ACC_GLOBAL classes), owned
     // derivative split mode (largest classes): primitive-chunk tasks and the
@@ -272,7 +284,7 @@ struct qx_handle {
     int wpq[QX_NCLS_ALL];        // warps per quartet, plain warp kernels
     int wpq_deriv[QX_NCLS_ALL];  // warps per quartet, derivative warp kernels
     int wpq_deriv2[QX_NCLS_ALL]; // second-derivative warp kernels (they run every primitive)
-    int rys_lp[QX_NCLS_ALL];     // Rys adjoint gradient: 1 = level-parallel table build (RK_GRADL)
+    int rys_param[QX_NCLS_ALL];  // the caller's parameter of the Rys derivative engine (reported back)
     int shard_rank = 0, shard_n = 1;
     int prim_stage = 0;  // split-mode VRR: primitive pairs staged per warp (2 x largest pair), 0 = off
     int wait_limit = 1 << 22;  // polls of the bounded waits on those staging copies
@@ -333,11 +345,15 @@ static int build_orders(qx_handle* h, const int2* const* lists) {
             const int2* L = lists[c];
             std::fill(pos.begin(), pos.end(), 0);
             key.resize((size_t)nq);
+            int most = 0;
             for (long long q = 0; q < nq; ++q) {
-                key[q] = (unsigned short)(NB - std::min(h->pairs[L[q].x].nprim * h->pairs[L[q].y].nprim, NB));
+                const int np = h->pairs[L[q].x].nprim * h->pairs[L[q].y].nprim;
+                most = std::max(most, np);
+                key[q] = (unsigned short)(NB - std::min(np, NB));
                 ++pos[key[q] + 1];
                 if (key[q] != key[0]) uniform[c] = 0;
             }
+            h->work[c].max_prims = most;
             if (uniform[c]) continue;
             for (int k = 0; k < NB; ++k) pos[k + 1] += pos[k];
             int* o = order.get() + off[c];
@@ -533,12 +549,10 @@ static int run_class(qx_handle* h, int cls, int mode, const int2* d_q, long long
         a.jk_dmax = h->d_dmax;
     }
     if (eng == ENG_RYS) {
-        RysArgs ra;
-        ra.e = a;
-        ra.rys = h->d_rys;
-        if (g_rys_launch[cls](ra, RK_PLAIN, mode, nq, s))
-            return fail(QX_E_UNSUPPORTED, "class (%d%d|%d%d): no Rys program", g_class_l[cls][0], g_class_l[cls][1],
-                        g_class_l[cls][2], g_class_l[cls][3]);
+        TileArgs ta;
+        ta.e = a;
+        ta.rys = h->d_rys;
+        g_tile_launch[cls](ta, TK_PLAIN, mode, nq, h->work[cls].max_prims, s);
     } else if (eng == ENG_COOP) {
         qx_launch_coop(g_coop_idx[cls], a, mode, s);
     } else if (eng == ENG_WARP || eng == ENG_WSPLIT) {
@@ -608,7 +622,7 @@ extern "C" int qx_initialize(int natom, const double* coords, int nshell, const 
     choose_engines(h);
     for (int c = 0; c < QX_NCLS_ALL; ++c) {
         h->wpq[c] = h->wpq_deriv[c] = h->wpq_deriv2[c] = 1;
-        h->rys_lp[c] = 0;
+        h->rys_param[c] = 0;
     }
     h->natom = natom;
     h->nshell = nshell;
@@ -1185,15 +1199,14 @@ static int run_rys_derk(qx_handle* h, int c, int k, double* out, const int* nu, 
         ra.slice_k = k;
         for (int i = 0; i < k; ++i) ra.slice_nu[i] = nu[i];
     }
-    if (g_rys_launch[c](ra, RK_DER1 + k - 1, 0, w.nq * ra.nchunk, cs)) return rys_unsupported(c, "derivative");
+    if (g_rys_launch[c](ra, RK_DER1 + k - 1, w.nq * ra.nchunk, cs)) return rys_unsupported(c, "derivative");
     QX_CUDA(cudaGetLastError());
     return QX_OK;
 }
 
-// Adjoint gradient (kind RK_GRAD) or Hessian-vector product (RK_HVP) of one
-// class through the Rys engine.
-static int run_rys_contract(qx_handle* h, int c, int kind, const double* D, double cj, double ck, double* grad,
-                            const double* dir, cudaStream_t cs) {
+// Hessian-vector product of one class through the Rys engine.
+static int run_rys_hvp(qx_handle* h, int c, const double* D, double cj, double ck, double* hv, const double* dir,
+                       cudaStream_t cs) {
     const ClassWork& w = h->work[c];
     if (!w.nq) return QX_OK;
     RysArgs ra;
@@ -1202,11 +1215,26 @@ static int run_rys_contract(qx_handle* h, int c, int kind, const double* D, doub
     ra.D = D;
     ra.cj = cj;
     ra.ck = ck;
-    ra.grad = grad;
+    ra.grad = hv;
     ra.dir = dir;
     ra.M = 3 * h->natom;
-    if (kind == RK_GRAD && h->rys_lp[c]) kind = RK_GRADL;
-    if (g_rys_launch[c](ra, kind, 0, w.nq, cs)) return rys_unsupported(c, kind == RK_HVP ? "Hessian" : "gradient");
+    if (g_rys_launch[c](ra, RK_HVP, w.nq, cs)) return rys_unsupported(c, "Hessian");
+    QX_CUDA(cudaGetLastError());
+    return QX_OK;
+}
+
+// Adjoint gradient of one class through the tile engine.
+static int run_tile_grad(qx_handle* h, int c, const double* D, double cj, double ck, double* grad, cudaStream_t cs) {
+    const ClassWork& w = h->work[c];
+    if (!w.nq) return QX_OK;
+    TileArgs ta;
+    ta.e = class_args(h, c, nullptr);
+    ta.rys = h->d_rys;
+    ta.D = D;
+    ta.cj = cj;
+    ta.ck = ck;
+    ta.grad = grad;
+    g_tile_launch[c](ta, TK_GRAD, 0, w.nq, w.max_prims, cs);
     QX_CUDA(cudaGetLastError());
     return QX_OK;
 }
@@ -1215,7 +1243,7 @@ static int run_rys_contract(qx_handle* h, int c, int kind, const double* D, doub
 static int run_deriv_class(qx_handle* h, int c, int mode, double* out, const double* D, double cj, double ck,
                            double* grad, int slice, cudaStream_t cs) {
     if (h->deriv_eng[c] == ENG_RYS) {
-        if (mode == QX_MODE_GRAD) return run_rys_contract(h, c, RK_GRAD, D, cj, ck, grad, nullptr, cs);
+        if (mode == QX_MODE_GRAD) return run_tile_grad(h, c, D, cj, ck, grad, cs);
         if (mode == QX_MODE_DER_DENSE) return run_rys_derk(h, c, 1, out, nullptr, cs);
         return run_rys_derk(h, c, 1, out, &slice, cs);
     }
@@ -1312,7 +1340,7 @@ static int run_all_deriv2(qx_handle* h, int mode, double* out, int slice, cudaSt
         if (!g_warp_deriv2[c]) {  // classes with d or f shells: the Rys engine
             int rc;
             if (mode == QX_MODE_HVP) {
-                rc = run_rys_contract(h, c, RK_HVP, D, cj, ck, hv, dir, cs);
+                rc = run_rys_hvp(h, c, D, cj, ck, hv, dir, cs);
             } else if (mode == QX_MODE_DER2_DENSE) {
                 rc = run_rys_derk(h, c, 2, out, nullptr, cs);
             } else {
@@ -1533,27 +1561,21 @@ extern "C" int qx_oei_deriv_core(qx_handle* h, int order, double* dS, double* dT
 }
 
 // ---------------------------------------------------------------- class info ---
-// Algorithmic FP64 FLOPs of one primitive quartet of the Rys programs (plain:
-// deriv = 0; adjoint gradient: deriv = 1), counted per step of qx_rys.cuh: the
-// 2n Chebyshev series (13 Clenshaw steps, 4 flops each), the 3n two-dimensional
-// tables (5 flops per entry), the transfer levels (2 per entry), the gradient's
-// four derivative tables (3 per entry) and the products (plain: 3 per component
-// and root; gradient: 22).
+// Algorithmic FP64 FLOPs of one primitive quartet of the tile programs (plain:
+// deriv = 0; adjoint gradient: deriv = 1), counted per step of qx_tile.cuh: the 2n
+// Chebyshev series (13 Clenshaw steps, 4 flops each), the 3n two-dimensional tables (5
+// flops per entry), and per f and root 2 flops per (e0|f0) value and 1 per (ex, ey) pair;
+// the gradient 6 per value, 5 per pair, and 2 for each of the lowered terms of the three
+// directions (bra and ket) and of E0.
 static double rys_prim_flops(const int* l, int deriv) {
-    const int L = l[0] + l[1] + l[2] + l[3];
-    const int A1 = l[0] + 1 + deriv, B1 = l[1] + 1 + deriv, C1 = l[2] + 1 + deriv, D1 = l[3] + 1;
-    const int NI = A1 + B1 - 1, NK = C1 + D1 - 1, NR = (L + deriv) / 2 + 1;
-    double ncomp = 1.0, sz0 = 1.0;
-    for (int i = 0; i < 4; ++i) {
-        ncomp *= (l[i] + 1) * (l[i] + 2) / 2;
-        sz0 *= l[i] + 1;
-    }
-    double f = 2.0 * NR * 52.0 + 3.0 * NR * NI * NK * 5.0;
-    for (int b = 1; b < B1; ++b) f += 3.0 * NR * (NI - b) * NK * 2.0;
-    for (int d = 1; d < D1; ++d) f += 3.0 * NR * A1 * B1 * (NK - d) * 2.0;
-    if (deriv) f += 3.0 * NR * 4.0 * sz0 * 3.0 + ncomp * NR * 22.0;
-    else f += ncomp * NR * 3.0;
-    return f;
+    const int L = l[0] + l[1] + l[2] + l[3], NR = (L + deriv) / 2 + 1;
+    const int HI = l[0] + l[1], NI = HI + 1, NK = l[2] + l[3] + 1;
+    auto hoff = [](int x) { return x * (x + 1) * (x + 2) / 6; };
+    const double NE = hoff(HI + 1) - hoff(l[0]), NF = hoff(l[2] + l[3] + 1) - hoff(l[2]);
+    const double pairs = (HI + 1) * (HI + 2) / 2;
+    const double f = 2.0 * NR * 52.0 + 3.0 * NR * NI * NK * 5.0;
+    if (!deriv) return f + NF * NR * (2.0 * NE + pairs);
+    return f + NF * NR * (6.0 * NE + 5.0 * pairs + 14.0 * (HI + 1));
 }
 
 extern "C" int qx_num_classes(void) { return QX_NCLS_ALL; }
@@ -1694,14 +1716,12 @@ extern "C" int qx_autotune(qx_handle* h, int what, void* stream) {
             if (g_has_wvrr[c]) cand.push_back({ENG_WVRR, 0});
             if (g_has_dsplit[c]) cand.push_back({ENG_DSPLIT, 0});
             if (g_der_idx[c] >= 0) cand.push_back({ENG_COOP, 0});
-            cand.push_back({ENG_RYS, 0});  // Rys, per-unit table build for small units
-            cand.push_back({ENG_RYS, 1});  // Rys, level-parallel table build
+            cand.push_back({ENG_RYS, 0});
             float best = 1e30f;
-            TuneCfg bc{h->deriv_eng[c], h->deriv_eng[c] == ENG_RYS ? h->rys_lp[c] : h->wpq_deriv[c]};
+            TuneCfg bc{h->deriv_eng[c], h->wpq_deriv[c]};
             for (const TuneCfg& t : cand) {
                 h->deriv_eng[c] = t.eng;
                 if (t.eng == ENG_WARP) h->wpq_deriv[c] = t.param;
-                if (t.eng == ENG_RYS) h->rys_lp[c] = t.param;
                 float ms = 0.f;
                 rc = time_config(s, e0, e1, &ms, [&] {
                     return run_deriv_class(h, c, QX_MODE_GRAD, nullptr, d_D, 1.0, -0.5, d_g, -1, s);
@@ -1714,7 +1734,6 @@ extern "C" int qx_autotune(qx_handle* h, int what, void* stream) {
             }
             h->deriv_eng[c] = bc.eng;
             if (bc.eng == ENG_WARP) h->wpq_deriv[c] = bc.param;
-            h->rys_lp[c] = bc.eng == ENG_RYS ? bc.param : 0;
         }
     }
     if (!rc) {
@@ -1733,9 +1752,8 @@ extern "C" int qx_autotune(qx_handle* h, int what, void* stream) {
 // Engine of one class chosen by the caller (tests, measurements): the autotuner's
 // choice made by hand.  plain / deriv: engine ids as qx_engine_config reports
 // them, -1 keeps the current one; pparam / dparam: log2 lanes per quartet
-// (straight-line) or warps per quartet (warp kernels); for the Rys derivative
-// engine dparam 0 or 1 picks the adjoint gradient's table build (per-unit for
-// small units, or level-parallel); ignored otherwise.
+// (straight-line) or warps per quartet (warp kernels); the Rys derivative engine
+// takes dparam 0 or 1, which select the same program; ignored otherwise.
 extern "C" int qx_set_engine(qx_handle* h, int cls, int plain, int pparam, int deriv, int dparam) {
     if (!h || cls < 0 || cls >= QX_NCLS_ALL) return fail(QX_E_INVALID, "qx_set_engine: bad handle or class");
     DeviceGuard g(h->device);
@@ -1783,7 +1801,7 @@ extern "C" int qx_set_engine(qx_handle* h, int cls, int plain, int pparam, int d
         if (!ok) return no("derivative", deriv);
         h->deriv_eng[cls] = deriv;
         if (deriv == ENG_WARP) h->wpq_deriv[cls] = dparam;
-        if (deriv == ENG_RYS) h->rys_lp[cls] = dparam;
+        if (deriv == ENG_RYS) h->rys_param[cls] = dparam;
     }
     return QX_OK;
 }
@@ -1836,7 +1854,7 @@ extern "C" int qx_engine_config(const qx_handle* h, int cls, int* cfg) {
     cfg[0] = h->plain_eng[cls];
     cfg[1] = h->plain_eng[cls] == ENG_SL ? h->work[cls].log2g : (h->plain_eng[cls] == ENG_WARP ? h->wpq[cls] : 0);
     cfg[2] = h->deriv_eng[cls];
-    cfg[3] = h->deriv_eng[cls] == ENG_WARP ? h->wpq_deriv[cls] : (h->deriv_eng[cls] == ENG_RYS ? h->rys_lp[cls] : 0);
+    cfg[3] = h->deriv_eng[cls] == ENG_WARP ? h->wpq_deriv[cls] : (h->deriv_eng[cls] == ENG_RYS ? h->rys_param[cls] : 0);
     return QX_OK;
 }
 
@@ -1915,7 +1933,7 @@ extern "C" int qx_deriv_tile(qx_handle* h, int cls, long long q0, long long q1, 
         ra.M = 3 * h->natom;
         ra.tile_E = E;
         ra.tile_images = images;
-        if (g_rys_launch[cls](ra, RK_GRADT, 0, a.nq, s)) return rys_unsupported(cls, "derivative-tile");
+        if (g_rys_launch[cls](ra, RK_GRADT, a.nq, s)) return rys_unsupported(cls, "derivative-tile");
     }
     QX_CUDA(cudaGetLastError());
     return QX_OK;

@@ -1,5 +1,6 @@
-// qx_rys.cuh -- Rys-quadrature engine: every class up to (ff|ff), and nuclear
-// derivatives of any order, through one looped design.
+// qx_rys.cuh -- Rys-quadrature engine for derivative tensors and Hessian-vector
+// products: every class up to (ff|ff), and nuclear derivatives of any order, through
+// one looped design.
 //
 // Method (published mathematics, written here):
 //   * A primitive integral is pref * sum_r w_r Ix(u_r) Iy(u_r) Iz(u_r), with
@@ -51,13 +52,11 @@ constexpr int RYS_TABLE_DOUBLES = QX_RYS_TAB_SIZE + 2 * QX_RYS_ASYM_SIZE;
 // Kinds of Rys programs: which centres are raised for derivatives, the
 // derivative order the quadrature must integrate, and the per-direction 1-D
 // derivative tables the products read.
-enum { RK_PLAIN = 0, RK_GRAD = 1, RK_HVP = 2, RK_GRADT = 3, RK_GRADL = 4, RK_DER1 = 11, RK_DER2 = 12,
-       RK_DER3 = 13, RK_DER4 = 14 };
-// The adjoint-gradient kinds: RK_GRADL is RK_GRAD with every unit's tables built
-// level by level over the team (the autotuner picks the faster build per class).
-QX_HD constexpr bool rys_is_grad(int kind) { return kind == RK_GRAD || kind == RK_GRADL; }
-// Epilogues of the plain kind (the derivative kinds have their own).
-enum { RMODE_DENSE = 0, RMODE_UNIQUE = 1, RMODE_SCHWARZ = 2, RMODE_JK = 3 };
+// The device kernel runs the Hessian-vector product, the gradient tile and the derivative
+// tensors; plain integrals and the adjoint gradient run in qx_tile.cuh, and their product
+// steps here serve the host check of the tables.
+enum { RK_PLAIN = 0, RK_GRAD = 1, RK_HVP = 2, RK_GRADT = 3, RK_DER1 = 11, RK_DER2 = 12, RK_DER3 = 13, RK_DER4 = 14 };
+QX_HD constexpr bool rys_is_grad(int kind) { return kind == RK_GRAD; }
 
 QX_HD constexpr int rys_binom(int n, int k) {
     if (k < 0 || k > n) return 0;
@@ -80,8 +79,6 @@ template <>
 struct RysKind<RK_GRAD> {  // A, B, C raised by one; dA, dB, dC formed in the products (D by invariance)
     static constexpr int ORD = 1, KA = 1, KB = 1, KC = 1, KD = 0, NOPS = 0;
 };
-template <>
-struct RysKind<RK_GRADL> : RysKind<RK_GRAD> {};
 template <>
 struct RysKind<RK_GRADT> {  // as RK_GRAD, but the 9 derivative integrals are written to a tile
     static constexpr int ORD = 1, KA = 1, KB = 1, KC = 1, KD = 0, NOPS = 0;
@@ -146,7 +143,7 @@ struct RysCls {
     static_assert((!RAW || SRAW < 1024) && SZ0 < 1024, "1-D table offsets exceed 10 bits");
     // one thread builds a whole (direction, root) unit -- 2-D table and both
     // transfers -- when the units keep at least a sixth of the team busy or are small
-    static constexpr bool SEQ = KIND != RK_GRADL && (6 * RB >= TS || SRAW <= 160);
+    static constexpr bool SEQ = 6 * RB >= TS || SRAW <= 160;
     // derivative tensors: multi-indices accumulated per pass over the primitives
     static constexpr int MG = NCPT >= 32 ? 1 : (32 / NCPT > 8 ? 8 : 32 / NCPT);
     // gradient tile: derivative coordinates (of the 9) accumulated per pass
@@ -156,7 +153,7 @@ struct RysCls {
 struct RysArgs {
     EriArgs e;
     const double* rys = nullptr;  // device table: QX_RYS_TAB | asymptotic y | asymptotic W
-    // adjoint gradient and Hessian-vector product
+    // Hessian-vector product
     const double* D = nullptr;
     double cj = 0.0, ck = 0.0;
     double* grad = nullptr;       // 3N output (atomic adds)
@@ -783,22 +780,6 @@ __device__ __forceinline__ double rys_team_sum(double v, double* red, int tid, i
     }
 }
 
-template <int TS, int TPB>
-__device__ __forceinline__ double rys_team_max(double v, double* red, int tid, int team) {
-    for (int off = 16; off > 0; off >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, off));
-    if constexpr (TS == 32) {
-        return v;
-    } else {
-        rys_team_sync<TS, TPB>(team);
-        if ((tid & 31) == 0) red[tid >> 5] = v;
-        rys_team_sync<TS, TPB>(team);
-        double s = 0.0;
-        if (tid == 0)
-            for (int w = 0; w < TS / 32; ++w) s = fmax(s, red[w]);
-        return s;
-    }
-}
-
 // Per primitive quartet: nodes/weights, then per root batch the tables and the
 // caller's product step `prod(nrb, e2)` (e2: twice the four exponents).
 template <class C, int KIND, int LA, int LB, int LC, int LD, class Prod>
@@ -838,7 +819,8 @@ __device__ __forceinline__ void rys_primitive(const RysArgs& ra, const PrimPair&
 
 template <int LA, int LB, int LC, int LD, int KIND>
 __global__ void __launch_bounds__(RysCls<LA, LB, LC, LD, KIND>::BS, RysCls<LA, LB, LC, LD, KIND>::MINB)
-    k_rys(RysArgs ra, int mode, long long nwork) {
+    k_rys(RysArgs ra, long long nwork) {
+    static_assert(KIND == RK_HVP || KIND == RK_GRADT || KIND >= RK_DER1, "plain integrals and the gradient: qx_tile.cuh");
     using C = RysCls<LA, LB, LC, LD, KIND>;
     constexpr int TS = C::TS, TPB = C::TPB, NCPT = C::NCPT;
     extern __shared__ double rys_sm[];
@@ -867,11 +849,7 @@ __global__ void __launch_bounds__(RysCls<LA, LB, LC, LD, KIND>::BS, RysCls<LA, L
         const PairInfo Q = a.pairs[pq.y];
         const int atoms[4] = {P.atom1, P.atom2, Q.atom1, Q.atom2};
         const bool s12 = P.s1 != P.s2, s34 = Q.s1 != Q.s2, sPQ = pq.x != pq.y;
-        if constexpr (KIND == RK_PLAIN) {
-            if (mode == RMODE_JK && jk_screened(a, pq, P, Q)) continue;  // team-uniform
-        } else {
-            if (atoms[0] == atoms[1] && atoms[0] == atoms[2] && atoms[0] == atoms[3]) continue;
-        }
+        if (atoms[0] == atoms[1] && atoms[0] == atoms[2] && atoms[0] == atoms[3]) continue;
         // derivative tensors: the work item's multi-indices
         int nm = 0;
         if constexpr (KIND >= RK_DER1) {
@@ -907,10 +885,10 @@ __global__ void __launch_bounds__(RysCls<LA, LB, LC, LD, KIND>::BS, RysCls<LA, L
         for (int j = 0; j < NCPT; ++j) {
             const int kc = tid + j * TS;
             offs[j] = kc < C::NCOMP ? rys_comp_offsets<C, LA, LB, LC, LD, C::RAW>(kc) : 0;
-            if constexpr (rys_is_grad(KIND) || KIND == RK_GRADT)
+            if constexpr (KIND == RK_GRADT)
                 exps[j] = kc < C::NCOMP ? rys_comp_exps<C, LA, LB, LC, LD>(kc) : 0;
             gam[j] = 0.0;
-            if constexpr (rys_is_grad(KIND) || KIND == RK_HVP) {
+            if constexpr (KIND == RK_HVP) {
                 if (kc < C::NCOMP) {
                     const int id = kc % C::ND, ic = (kc / C::ND) % C::NC, ib = (kc / (C::ND * C::NC)) % C::NB,
                               ia = kc / (C::ND * C::NC * C::NB);
@@ -937,47 +915,7 @@ __global__ void __launch_bounds__(RysCls<LA, LB, LC, LD, KIND>::BS, RysCls<LA, L
             if (still) continue;
         }
         const int nk = Q.nprim, ntot = P.nprim * nk;
-        if constexpr (KIND == RK_PLAIN) {
-            double acc[NCPT];
-#pragma unroll
-            for (int j = 0; j < NCPT; ++j) acc[j] = 0.0;
-            for (int t = 0; t < ntot; ++t) {
-                const int i = t / nk, jj = t - i * nk;
-                rys_primitive<C, KIND, LA, LB, LC, LD>(ra, a.prims[P.prim_off + i], a.prims[Q.prim_off + jj], P, Q,
-                                                        uw, U, O, w9, tid, team, [&](int nrb, const double*) {
-#pragma unroll
-                    for (int j = 0; j < NCPT; ++j)
-                        if (tid + j * TS < C::NCOMP) acc[j] += rys_prod_plain<C>(U, nrb, offs[j]);
-                });
-            }
-            if (mode == RMODE_SCHWARZ) {
-                double mx = 0.0;
-#pragma unroll
-                for (int j = 0; j < NCPT; ++j) {
-                    const int kc = tid + j * TS;
-                    if (kc < C::NCOMP && kc / (C::NC * C::ND) == kc % (C::NC * C::ND)) mx = fmax(mx, fabs(acc[j]));
-                }
-                mx = rys_team_max<TS, TPB>(mx, red, tid, team);
-                if (tid == 0) a.out[pq.x] = mx;
-                continue;
-            }
-#pragma unroll
-            for (int j = 0; j < NCPT; ++j) {
-                const int kc = tid + j * TS;
-                if (kc >= C::NCOMP) continue;
-                if (mode == RMODE_UNIQUE) {
-                    a.out[a.base + (long long)kc * a.nq + qi] = acc[j];
-                    continue;
-                }
-                const int id = kc % C::ND, ic = (kc / C::ND) % C::NC, ib = (kc / (C::ND * C::NC)) % C::NB,
-                          ia = kc / (C::ND * C::NC * C::NB);
-                const long long ii = P.bf1 + ia, jj = P.bf2 + ib, kk = Q.bf1 + ic, ll = Q.bf2 + id;
-                if (mode == RMODE_JK)
-                    jk_images(a.out, a.out2, a.dens, n, ii, jj, kk, ll, s12, s34, sPQ, acc[j]);
-                else
-                    dense_images(a.out, n, ii, jj, kk, ll, s12, s34, sPQ, acc[j]);
-            }
-        } else if constexpr (KIND == RK_GRADT) {
+        if constexpr (KIND == RK_GRADT) {
             // the first-derivative integrals of the quartet, summed over primitives in
             // registers (GG coordinates per pass), then added into the tile: centre X's
             // block to its atom's rows, minus the sum to the D centre's atom
@@ -1013,7 +951,7 @@ __global__ void __launch_bounds__(RysCls<LA, LB, LC, LD, KIND>::BS, RysCls<LA, L
                     }
                 }
             }
-        } else if constexpr (rys_is_grad(KIND) || KIND == RK_HVP) {
+        } else if constexpr (KIND == RK_HVP) {
             double g[9];
 #pragma unroll
             for (int b = 0; b < 9; ++b) g[b] = 0.0;
@@ -1023,12 +961,7 @@ __global__ void __launch_bounds__(RysCls<LA, LB, LC, LD, KIND>::BS, RysCls<LA, L
                                                         uw, U, O, w9, tid, team, [&](int nrb, const double* e2) {
 #pragma unroll
                     for (int j = 0; j < NCPT; ++j)
-                        if (tid + j * TS < C::NCOMP) {
-                            if constexpr (rys_is_grad(KIND))
-                                rys_prod_grad<C>(U, nrb, offs[j], exps[j], e2, gam[j], g);
-                            else
-                                rys_prod_hvp<C>(O, nrb, offs[j], gam[j], g);
-                        }
+                        if (tid + j * TS < C::NCOMP) rys_prod_hvp<C>(O, nrb, offs[j], gam[j], g);
                 });
             }
 #pragma unroll
@@ -1090,7 +1023,7 @@ __global__ void __launch_bounds__(RysCls<LA, LB, LC, LD, KIND>::BS, RysCls<LA, L
 // Host launcher of one class and kind; returns false when the class's tables do
 // not fit shared memory for this kind.
 template <int LA, int LB, int LC, int LD, int KIND>
-bool launch_rys(const RysArgs& ra, int mode, long long nwork, cudaStream_t s) {
+bool launch_rys(const RysArgs& ra, long long nwork, cudaStream_t s) {
     using C = RysCls<LA, LB, LC, LD, KIND>;
     if constexpr (!C::FITS) {
         return false;
@@ -1108,7 +1041,7 @@ bool launch_rys(const RysArgs& ra, int mode, long long nwork, cudaStream_t s) {
         long long nb = (nwork + C::TPB - 1) / C::TPB;
         const long long cap = 148LL * per_sm * 8;
         if (nb > cap) nb = cap;
-        k<<<(unsigned)nb, C::BS, C::SMEM, s>>>(ra, mode, nwork);
+        k<<<(unsigned)nb, C::BS, C::SMEM, s>>>(ra, nwork);
         return true;
     }
 }
