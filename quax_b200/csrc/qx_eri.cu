@@ -1182,6 +1182,13 @@ static int rys_unsupported(int c, const char* what) {
                 g_class_l[c][0], g_class_l[c][1], g_class_l[c][2], g_class_l[c][3], what);
 }
 
+// Work items that share a quartet's primitives in the Rys kernels: a team walks its
+// primitives one after another (up to 4,096 of them), so few quartets would leave most
+// of the GPU idle behind the largest one.  The outputs are sums of atomics either way.
+static int rys_parts(long long items, int max_prims) {
+    return (int)std::min<long long>(148LL * 32 / items + 1, std::max(1, max_prims / 4));
+}
+
 // Derivative tensor of order k (1..4) of one class through the Rys engine:
 // dense (nu == nullptr; slot = the reference's rank of the sorted nuclear indices
 // over M = 3N) or the one slice of the sorted nuclear indices nu[0..k).
@@ -1199,7 +1206,8 @@ static int run_rys_derk(qx_handle* h, int c, int k, double* out, const int* nu, 
         ra.slice_k = k;
         for (int i = 0; i < k; ++i) ra.slice_nu[i] = nu[i];
     }
-    if (g_rys_launch[c](ra, RK_DER1 + k - 1, w.nq * ra.nchunk, cs)) return rys_unsupported(c, "derivative");
+    ra.parts = rys_parts(w.nq * ra.nchunk, w.max_prims);
+    if (g_rys_launch[c](ra, RK_DER1 + k - 1, w.nq * ra.nchunk * ra.parts, cs)) return rys_unsupported(c, "derivative");
     QX_CUDA(cudaGetLastError());
     return QX_OK;
 }
@@ -1218,7 +1226,8 @@ static int run_rys_hvp(qx_handle* h, int c, const double* D, double cj, double c
     ra.grad = hv;
     ra.dir = dir;
     ra.M = 3 * h->natom;
-    if (g_rys_launch[c](ra, RK_HVP, w.nq, cs)) return rys_unsupported(c, "Hessian");
+    ra.parts = rys_parts(w.nq, w.max_prims);
+    if (g_rys_launch[c](ra, RK_HVP, w.nq * ra.parts, cs)) return rys_unsupported(c, "Hessian");
     QX_CUDA(cudaGetLastError());
     return QX_OK;
 }

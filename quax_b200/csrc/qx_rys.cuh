@@ -112,8 +112,9 @@ struct RysCls {
     static constexpr int NOPS = K::NOPS;
     static constexpr int UOPS = NOPS * SZ0;
     // team size: about 12 components per thread (8 for the gradient tile, which
-    // keeps 9 sums per component), 32..256 threads
-    static constexpr int TS0 = KIND == RK_GRADT ? (NCOMP + 7) / 8 : (NCOMP + 11) / 12;
+    // keeps 9 sums per component; 6 for the derivative tensors, which build the tables
+    // once per pass over the multi-indices), 32..256 threads
+    static constexpr int TS0 = KIND == RK_GRADT ? (NCOMP + 7) / 8 : (KIND >= RK_DER1 ? (NCOMP + 5) / 6 : (NCOMP + 11) / 12);
     static constexpr int TS1 = TS0 <= 32 ? 32 : TS0 <= 64 ? 64 : TS0 <= 128 ? 128 : 256;
     static constexpr int HDR = RYS_HDR + (KIND >= RK_DER1 ? RYS_DERK_HDR : 0);
     static constexpr int PER_ROOT = 3 * (USZ + UOPS);
@@ -145,7 +146,7 @@ struct RysCls {
     // transfers -- when the units keep at least a sixth of the team busy or are small
     static constexpr bool SEQ = 6 * RB >= TS || SRAW <= 160;
     // derivative tensors: multi-indices accumulated per pass over the primitives
-    static constexpr int MG = NCPT >= 32 ? 1 : (32 / NCPT > 8 ? 8 : 32 / NCPT);
+    static constexpr int MG = NCPT >= 72 ? 1 : (72 / NCPT > 16 ? 16 : 72 / NCPT);
     // gradient tile: derivative coordinates (of the 9) accumulated per pass
     static constexpr int GG = NCPT * 9 <= 72 ? 9 : (72 / NCPT < 1 ? 1 : 72 / NCPT);
 };
@@ -161,7 +162,8 @@ struct RysArgs {
     // derivative tensors (RK_DERk): dense (slice_k == 0) or one slice
     int M = 0;                    // 3N
     int chunk = 1;                // multi-indices per work item
-    int nchunk = 1;               // work items per quartet
+    int nchunk = 1;               // multi-index chunks per quartet
+    int parts = 1;                // work items that share a quartet's primitives (and chunk)
     int slice_k = 0;              // 0: dense; else the slice's order (== k)
     int slice_nu[4] = {0, 0, 0, 0};  // the slice's sorted nuclear indices
     // first-derivative tile (RK_DER1 only): out is a (3N, tile_E) row-major
@@ -435,84 +437,103 @@ QX_HD inline double rys_op_value(const RysPrim& s, double* U, int u, const int* 
     return v;
 }
 
+// First and second derivatives of a unit at the unraised point with raw offset o and
+// indices n[X] (centres A, B, C, D): d1(X), d2(X, X), d2(X, Y) from the factors of
+// d g_i = e2 g_{i+1} - i g_{i-1}.
+template <class C>
+struct RysDerivs {
+    const double* T;  // the unit's raw table at o
+    const double* e2;
+    int n[4];
+    QX_HD static constexpr int stride(int X) { return X == 0 ? C::B1 * C::D1 * C::NK : (X == 1 ? C::D1 * C::NK : (X == 2 ? 1 : C::NK)); }
+    template <int X>
+    QX_HD double d1() const {
+        constexpr int S = stride(X);
+        double r = e2[X] * T[S];
+        if (n[X]) r -= n[X] * T[-S];
+        return r;
+    }
+    template <int X, int Y>
+    QX_HD double d2() const {
+        constexpr int S = stride(X), Q = stride(Y);
+        if constexpr (X == Y) {
+            const int i = n[X];
+            double r = e2[X] * e2[X] * T[2 * S];
+            r -= e2[X] * (2 * i + 1) * T[0];
+            if (i >= 2) r += (double)(i * (i - 1)) * T[-2 * S];
+            return r;
+        } else {
+            double r = e2[X] * e2[Y] * T[S + Q];
+            if (n[Y]) r -= e2[X] * n[Y] * T[S - Q];
+            if (n[X]) r -= n[X] * e2[Y] * T[Q - S];
+            if (n[X] && n[Y]) r += (double)(n[X] * n[Y]) * T[-S - Q];
+            return r;
+        }
+    }
+};
+
 // Op tables of the derivative kinds: O holds per unit NOPS tables of SZ0
 // entries [a][b][c][d] (unraised extents).  RK_DERk: every (ka, kb, kc, kd)
 // with sum <= k in rys_op_rank order; RK_HVP: I, dA, dB, dC, V, dA V, dB V, dC V
-// with V = sum_X w_X dX along the direction w (per unit direction:
-// w9[3 * X + direction]).
+// with V = sum_X w_X dX along the direction (per unit direction: w9[3 * X +
+// direction]).  Up to second order a thread forms all ops of an element, so the raw
+// entries they share are read once and the indices decoded once (one op per thread,
+// with the orders unranked at run time, took most of an order-2 program's time);
+// above, one op per thread.
 template <class C, int KIND, int LA, int LB, int LC, int LD>
 QX_HD inline void rys_phase_ops(const RysPrim& s, int nrb, double* U, double* O, const double* w9, int tid, int nth) {
     constexpr int per = C::NOPS * C::SZ0;
-    for (int e = tid; e < 3 * nrb * per; e += nth) {
-        const int u = e / per;
-        const int rest = e - u * per, op = rest / C::SZ0, el = rest - op * C::SZ0;
-        const int d = el % (LD + 1), c = (el / (LD + 1)) % (LC + 1), b = (el / ((LD + 1) * (LC + 1))) % (LB + 1),
-                  a = el / ((LD + 1) * (LC + 1) * (LB + 1));
-        double v;
-        if constexpr (KIND == RK_HVP) {
-            // first and second derivatives on A, B, C in closed form: per centre the
-            // index shifts by +-1 (+-2 for a repeated centre) with the factors of
-            // d g_i = e2 g_{i+1} - i g_{i-1}
-            const int x = u % 3;
-            const int idx0[3] = {a, b, c};
-            auto R = [&](const int* ix) { return rys_gk<C>(U, u, ix[0], ix[1], d, ix[2]); };
-            auto d1 = [&](int X) {  // dX I
-                int ix[3] = {a, b, c};
-                ix[X] += 1;
-                double r = s.e2[X] * R(ix);
-                if (idx0[X]) {
-                    ix[X] -= 2;
-                    r -= idx0[X] * R(ix);
-                }
-                return r;
-            };
-            auto d2 = [&](int X, int Y) {  // dX dY I
-                int ix[3] = {a, b, c};
-                if (X == Y) {
-                    const int i = idx0[X];
-                    ix[X] = i + 2;
-                    double r = s.e2[X] * s.e2[X] * R(ix);
-                    ix[X] = i;
-                    r -= s.e2[X] * (2 * i + 1) * R(ix);
-                    if (i >= 2) {
-                        ix[X] = i - 2;
-                        r += (double)(i * (i - 1)) * R(ix);
-                    }
-                    return r;
-                }
-                double r = 0.0;
-                for (int sx = 0; sx < 2; ++sx)
-                    for (int sy = 0; sy < 2; ++sy) {
-                        const int ixx = idx0[X] + (sx ? -1 : 1), iyy = idx0[Y] + (sy ? -1 : 1);
-                        if (ixx < 0 || iyy < 0) continue;
-                        const double cf = (sx ? -(double)idx0[X] : s.e2[X]) * (sy ? -(double)idx0[Y] : s.e2[Y]);
-                        int jx[3] = {a, b, c};
-                        jx[X] = ixx;
-                        jx[Y] = iyy;
-                        r += cf * R(jx);
-                    }
-                return r;
-            };
-            if (op == 0) {
-                v = R(idx0);
-            } else if (op < 4) {
-                v = d1(op - 1);
-            } else if (op == 4) {
-                v = w9[x] * d1(0) + w9[3 + x] * d1(1) + w9[6 + x] * d1(2);
+    if constexpr (KIND == RK_HVP || C::K::ORD <= 2) {
+        for (int e = tid; e < 3 * nrb * C::SZ0; e += nth) {
+            const int u = e / C::SZ0, el = e - u * C::SZ0;
+            const int d = el % (LD + 1), c = (el / (LD + 1)) % (LC + 1), b = (el / ((LD + 1) * (LC + 1))) % (LB + 1),
+                      a = el / ((LD + 1) * (LC + 1) * (LB + 1));
+            const RysDerivs<C> q{&rys_gk<C>(U, u, a, b, d, c), s.e2, {a, b, c, d}};
+            double* o = O + (size_t)u * per + el;
+            auto put = [&](int op, double v) { o[op * C::SZ0] = v; };
+            if constexpr (KIND == RK_HVP) {
+                const int x = u % 3;
+                const double wA = w9[x], wB = w9[3 + x], wC = w9[6 + x];
+                const double dA = q.template d1<0>(), dB = q.template d1<1>(), dC = q.template d1<2>();
+                const double AB = q.template d2<0, 1>(), AC = q.template d2<0, 2>(), BC = q.template d2<1, 2>();
+                put(0, q.T[0]);
+                put(1, dA);
+                put(2, dB);
+                put(3, dC);
+                put(4, wA * dA + wB * dB + wC * dC);
+                put(5, wA * q.template d2<0, 0>() + wB * AB + wC * AC);
+                put(6, wA * AB + wB * q.template d2<1, 1>() + wC * BC);
+                put(7, wA * AC + wB * BC + wC * q.template d2<2, 2>());
+            } else if constexpr (C::K::ORD == 1) {
+                put(0, q.T[0]);
+                put(1, q.template d1<3>());
+                put(2, q.template d1<2>());
+                put(3, q.template d1<1>());
+                put(4, q.template d1<0>());
             } else {
-                const int Y = op - 5;
-                v = w9[x] * d2(0, Y) + w9[3 + x] * d2(1, Y) + w9[6 + x] * d2(2, Y);
+                put(0, q.T[0]);
+                put(1, q.template d1<3>());
+                put(2, q.template d2<3, 3>());
+                put(3, q.template d1<2>());
+                put(4, q.template d2<2, 3>());
+                put(5, q.template d2<2, 2>());
+                put(6, q.template d1<1>());
+                put(7, q.template d2<1, 3>());
+                put(8, q.template d2<1, 2>());
+                put(9, q.template d2<1, 1>());
+                put(10, q.template d1<0>());
+                put(11, q.template d2<0, 3>());
+                put(12, q.template d2<0, 2>());
+                put(13, q.template d2<0, 1>());
+                put(14, q.template d2<0, 0>());
             }
-        } else if constexpr (C::K::ORD == 1) {
-            // order 1, all four centres raised: ops in rys_op_rank order are
-            // I, dD, dC, dB, dA, in closed form
-            auto R = [&](int ia, int ib, int ic, int id) { return rys_gk<C>(U, u, ia, ib, id, ic); };
-            if (op == 0) v = R(a, b, c, d);
-            else if (op == 1) v = s.e2[3] * R(a, b, c, d + 1) - (d ? d * R(a, b, c, d - 1) : 0.0);
-            else if (op == 2) v = s.e2[2] * R(a, b, c + 1, d) - (c ? c * R(a, b, c - 1, d) : 0.0);
-            else if (op == 3) v = s.e2[1] * R(a, b + 1, c, d) - (b ? b * R(a, b - 1, c, d) : 0.0);
-            else v = s.e2[0] * R(a + 1, b, c, d) - (a ? a * R(a - 1, b, c, d) : 0.0);
-        } else {
+        }
+    } else {
+        for (int e = tid; e < 3 * nrb * per; e += nth) {
+            const int u = e / per;
+            const int rest = e - u * per, op = rest / C::SZ0, el = rest - op * C::SZ0;
+            const int d = el % (LD + 1), c = (el / (LD + 1)) % (LC + 1), b = (el / ((LD + 1) * (LC + 1))) % (LB + 1),
+                      a = el / ((LD + 1) * (LC + 1) * (LB + 1));
             constexpr int K = C::K::ORD;
             // unrank op within tuples of sum <= K (lexicographic)
             int k[4];
@@ -530,9 +551,8 @@ QX_HD inline void rys_phase_ops(const RysPrim& s, int nrb, double* U, double* O,
                 left -= val;
             }
             k[3] = r;
-            v = rys_op_value<C>(s, U, u, k, a, b, c, d);
+            O[(size_t)u * per + op * C::SZ0 + el] = rys_op_value<C>(s, U, u, k, a, b, c, d);
         }
-        O[(size_t)u * per + op * C::SZ0 + el] = v;
     }
 }
 
@@ -837,11 +857,13 @@ __global__ void __launch_bounds__(RysCls<LA, LB, LC, LD, KIND>::BS, RysCls<LA, L
     const long long n = a.n;
     const long long nteams = (long long)gridDim.x * TPB;
     for (long long w = (long long)blockIdx.x * TPB + team; w < nwork; w += nteams) {
-        long long qi = w;
+        long long qi = w / ra.parts;
+        const int part = (int)(w - qi * ra.parts);
         int ch = 0;
         if constexpr (KIND >= RK_DER1) {
-            qi = w / ra.nchunk;
-            ch = (int)(w - qi * ra.nchunk);
+            const long long q = qi;
+            qi = q / ra.nchunk;
+            ch = (int)(q - qi * ra.nchunk);
         }
         qi = list_index(a, qi);
         const int2 pq = a.quartets[qi];
@@ -850,6 +872,7 @@ __global__ void __launch_bounds__(RysCls<LA, LB, LC, LD, KIND>::BS, RysCls<LA, L
         const int atoms[4] = {P.atom1, P.atom2, Q.atom1, Q.atom2};
         const bool s12 = P.s1 != P.s2, s34 = Q.s1 != Q.s2, sPQ = pq.x != pq.y;
         if (atoms[0] == atoms[1] && atoms[0] == atoms[2] && atoms[0] == atoms[3]) continue;
+        if (part >= P.nprim * Q.nprim) continue;  // team-uniform, as the test above
         // derivative tensors: the work item's multi-indices
         int nm = 0;
         if constexpr (KIND >= RK_DER1) {
@@ -926,7 +949,7 @@ __global__ void __launch_bounds__(RysCls<LA, LB, LC, LD, KIND>::BS, RysCls<LA, L
                 for (int j = 0; j < NCPT; ++j)
 #pragma unroll
                     for (int g = 0; g < GG; ++g) acc[j][g] = 0.0;
-                for (int t = 0; t < ntot; ++t) {
+                for (int t = part; t < ntot; t += ra.parts) {
                     const int i = t / nk, jj = t - i * nk;
                     rys_primitive<C, KIND, LA, LB, LC, LD>(ra, a.prims[P.prim_off + i], a.prims[Q.prim_off + jj], P,
                                                             Q, uw, U, O, w9, tid, team, [&](int nrb, const double* e2) {
@@ -955,7 +978,7 @@ __global__ void __launch_bounds__(RysCls<LA, LB, LC, LD, KIND>::BS, RysCls<LA, L
             double g[9];
 #pragma unroll
             for (int b = 0; b < 9; ++b) g[b] = 0.0;
-            for (int t = 0; t < ntot; ++t) {
+            for (int t = part; t < ntot; t += ra.parts) {
                 const int i = t / nk, jj = t - i * nk;
                 rys_primitive<C, KIND, LA, LB, LC, LD>(ra, a.prims[P.prim_off + i], a.prims[Q.prim_off + jj], P, Q,
                                                         uw, U, O, w9, tid, team, [&](int nrb, const double* e2) {
@@ -985,7 +1008,7 @@ __global__ void __launch_bounds__(RysCls<LA, LB, LC, LD, KIND>::BS, RysCls<LA, L
                 for (int j = 0; j < NCPT; ++j)
 #pragma unroll
                     for (int mm = 0; mm < MG; ++mm) acc[j][mm] = 0.0;
-                for (int t = 0; t < ntot; ++t) {
+                for (int t = part; t < ntot; t += ra.parts) {
                     const int i = t / nk, jj = t - i * nk;
                     rys_primitive<C, KIND, LA, LB, LC, LD>(ra, a.prims[P.prim_off + i], a.prims[Q.prim_off + jj], P,
                                                             Q, uw, U, O, w9, tid, team, [&](int nrb, const double*) {

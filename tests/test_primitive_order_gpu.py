@@ -10,8 +10,9 @@ blocks of the same shells to 1e-13 of the block's scale (split-mode sums meet in
 order)."""
 import numpy as np
 import pytest
+import torch
 
-from quax_b200.basis import SyntheticSpec, synthetic_molecule
+from quax_b200.basis import Basis, Shell, SyntheticSpec, synthetic_molecule
 from quax_b200.integrals.engine import EriEngine
 
 pytestmark = pytest.mark.gpu
@@ -33,6 +34,26 @@ def test_dropped_primitives(oracle_lib, tol):
     assert used < full
     G = eng.eri().cpu().numpy()
     assert np.abs(G - oracle_lib.compute_2e_int(ob, tol)).max() < 1e-12
+
+
+def test_dropped_primitives_second_derivatives():
+    """Hessian-vector products of s and p shells, whose programs cancel sums of (2 alpha)^2
+    weights, do not depend on the primitives a threshold drops.  Shells with a diffuse and
+    tight primitives on close atoms, so that both thresholds keep every quartet: the same
+    sums in the same order but for the atomics, 1e-12 of the largest entry (grouping them
+    otherwise moved five atoms' product by 2.8e-9)."""
+    xyz = np.array([[0.0, 0.0, 0.0], [0.0, 1.1, 2.6], [2.4, 0.4, -1.3]])
+    exps, coef = np.array([3000.0, 400.0, 60.0, 9.0, 0.3]), np.array([0.1, 0.2, 0.4, 0.6, 1.0])
+    b = Basis([Shell(l, exps, coef, x.copy(), a) for a, x in enumerate(xyz) for l in (0, 0, 1)], 3)
+    n = b.nbf()
+    rng = np.random.default_rng(3)
+    C = rng.normal(0.0, 1.0 / np.sqrt(n), size=(n, max(1, n // 4)))
+    D, v = torch.from_numpy(C @ C.T).cuda(), torch.from_numpy(rng.normal(size=3 * b.natom)).cuda()
+    e = [EriEngine(b, tol) for tol in (1e-12, 1e-60)]
+    assert e[0].unique_quartets() == e[1].unique_quartets()
+    assert sum(c["prims"] for c in e[0].class_info()) < sum(c["prims"] for c in e[1].class_info())
+    h = [x.grad_adjoint_jvp(D, v, 2.0, -1.0).cpu().numpy() for x in e]
+    assert np.abs(h[0] - h[1]).max() < 1e-12 * np.abs(h[1]).max()
 
 
 def test_layout_of_views():
