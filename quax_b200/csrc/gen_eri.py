@@ -1146,17 +1146,18 @@ def gen_rys(here, lmax_os):
 
 def gen_tile(here):
     """One translation unit per class up to RYS_LMAX with the tile engine's launcher
-    qx_launch_tile_<id>(args, kind, mode, nquartets, largest primitive count, stream)."""
+    qx_launch_tile_<id>(args, kind, mode, nquartets, primitive quartets, the largest
+    quartet's, counts above powers of two, stream)."""
     qc = quartet_classes(RYS_LMAX)
     for i, (a, b, c, d) in enumerate(qc):
         L = ["// Generated by quax_b200/csrc/gen_eri.py -- do not edit by hand.",
              f"// Tile-engine launchers of class ({a}{b}|{c}{d}).",
              '#include "../qx_tile.cuh"',
-             f"void qx_launch_tile_{i:02d}(qx::TileArgs& ta, int kind, int mode, long long nq, int max_prims, "
-             "cudaStream_t s) {"]
+             f"void qx_launch_tile_{i:02d}(qx::TileArgs& ta, int kind, int mode, long long nq, long long prims, "
+             "int max_prims, const int* prefix, cudaStream_t s) {"]
         for k in ("TK_PLAIN", "TK_GRAD"):
             L.append(f"    if (kind == qx::{k}) return qx::launch_tile<qx::TileCls<{a}, {b}, {c}, {d}, qx::{k}>>"
-                     "(ta, mode, nq, max_prims, s);")
+                     "(ta, mode, nq, prims, max_prims, prefix, s);")
         L += ["}"]
         with _Out(os.path.join(here, "gen", f"k_tile_{i:02d}.cu")) as f:
             f.write("\n".join(L) + "\n")

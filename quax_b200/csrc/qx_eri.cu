@@ -103,8 +103,10 @@ QX_FOR_EACH_CLASS_ALL(QX_DECL_RYS)
 #undef QX_DECL_RYS
 static RysLaunch g_rys_launch[QX_NCLS_ALL];
 // Tile-engine launchers, one per class (gen/k_tile_<id>.cu).
-typedef void (*TileLaunch)(qx::TileArgs&, int kind, int mode, long long nq, int max_prims, cudaStream_t);
-#define QX_DECL_TILE(id, a, b, c, d) void qx_launch_tile_##id(qx::TileArgs&, int, int, long long, int, cudaStream_t);
+typedef void (*TileLaunch)(qx::TileArgs&, int kind, int mode, long long nq, long long prims, int max_prims,
+                           const int* prefix, cudaStream_t);
+#define QX_DECL_TILE(id, a, b, c, d) \
+    void qx_launch_tile_##id(qx::TileArgs&, int, int, long long, long long, int, const int*, cudaStream_t);
 QX_FOR_EACH_CLASS_ALL(QX_DECL_TILE)
 #undef QX_DECL_TILE
 static TileLaunch g_tile_launch[QX_NCLS_ALL];
@@ -216,6 +218,7 @@ struct ClassWork {
     long long unique_base = 0;
     long long prims = 0;       // primitive quartets of the class
     int max_prims = 0;         // of its largest quartet
+    int prefix[TILE_SEGS] = {};  // with an order: quartets with more than 2^k primitives
     int log2g = 0;             // lanes per quartet = 2^log2g
     double* scratch = nullptr; // global accumulators (ACC_GLOBAL classes), owned
     // derivative split mode (largest classes): primitive-chunk tasks and the
@@ -263,7 +266,8 @@ struct qx_handle {
     PairInfo* d_pairs = nullptr;
     int* d_orders = nullptr;  // the classes' processing orders
     // pair records and primitive pairs with none dropped, for the second-derivative
-    // programs of the s and p classes (null: nothing was dropped from their pairs)
+    // programs of the s and p classes (null: nothing was dropped from their pairs); behind
+    // the others in the same allocations
     PairInfo* d_pairs_all = nullptr;
     PrimPair* d_prims_all = nullptr;
     double* d_boys = nullptr;
@@ -280,7 +284,8 @@ struct qx_handle {
     cudaEvent_t start = nullptr;
     int order[QX_NCLS_ALL];  // classes by decreasing primitive work
     int plain_eng[QX_NCLS_ALL];
-    int deriv_eng[QX_NCLS_ALL];
+    int deriv_eng[QX_NCLS_ALL];  // derivative tensors
+    int grad_eng[QX_NCLS_ALL];   // adjoint gradient
     int wpq[QX_NCLS_ALL];        // warps per quartet, plain warp kernels
     int wpq_deriv[QX_NCLS_ALL];  // warps per quartet, derivative warp kernels
     int wpq_deriv2[QX_NCLS_ALL]; // second-derivative warp kernels (they run every primitive)
@@ -356,6 +361,7 @@ static int build_orders(qx_handle* h, const int2* const* lists) {
             h->work[c].max_prims = most;
             if (uniform[c]) continue;
             for (int k = 0; k < NB; ++k) pos[k + 1] += pos[k];
+            for (int k = 0; k < TILE_SEGS; ++k) h->work[c].prefix[k] = pos[NB - std::min(1 << k, NB)];
             int* o = order.get() + off[c];
             for (long long q = 0; q < nq; ++q) o[pos[key[q]]++] = (int)q;
         }
@@ -461,7 +467,7 @@ static void choose_engines(qx_handle* h) {
     const char* de = std::getenv("QX_DERIV_ENGINE");
     for (int c = 0; c < QX_NCLS_ALL; ++c) {
         if (!has_os(c)) {  // f shells: the Rys engine only
-            h->plain_eng[c] = h->deriv_eng[c] = ENG_RYS;
+            h->plain_eng[c] = h->deriv_eng[c] = h->grad_eng[c] = ENG_RYS;
             continue;
         }
         int p;
@@ -475,9 +481,12 @@ static void choose_engines(qx_handle* h) {
             if (!std::strcmp(pe, "coop") && g_class_coop[c]) p = ENG_COOP;
             if (!std::strcmp(pe, "wsplit") && g_has_pvrr[c]) p = ENG_WSPLIT;
         }
-        // split VRR with the warp HRR where the class has it, else the split VRR with
-        // the cooperative HRR for L >= 6 (measured on the 10-atom workload); the
-        // autotuner settles each class per molecule
+        // tensors: split VRR with the warp HRR where the class has it, else the split VRR
+        // with the cooperative HRR for L >= 6 (measured on the 10-atom workload).  The
+        // adjoint gradient: the tile kernels from L = 4 on -- ten atoms, sum over those
+        // classes 24.0 ms with the split programs, 13.6 with the tiles; below, 4.9 against
+        // 10.0 (a block's set-up and its barriers for a few values).  The autotuner settles
+        // each class per molecule
         const int L = g_class_l[c][0] + g_class_l[c][1] + g_class_l[c][2] + g_class_l[c][3];
         int d = g_has_dsplit[c] ? ENG_DSPLIT
                 : (g_has_wvrr[c] && (L >= 6 || !g_has_warp_deriv[c])) ? ENG_WVRR
@@ -487,6 +496,7 @@ static void choose_engines(qx_handle* h) {
         if (de && !std::strcmp(de, "dsplit") && g_has_dsplit[c]) d = ENG_DSPLIT;
         h->plain_eng[c] = p;
         h->deriv_eng[c] = d;
+        h->grad_eng[c] = L >= 4 && !de ? (int)ENG_RYS : d;
     }
 }
 
@@ -496,8 +506,6 @@ static void free_handle(qx_handle* h) {
     if (!h) return;
     cudaFree(h->d_prims);
     cudaFree(h->d_orders);
-    cudaFree(h->d_pairs_all);
-    cudaFree(h->d_prims_all);
     cudaFree(h->d_pairs);
     cudaFree(h->d_boys);
     cudaFree(h->d_err);
@@ -552,7 +560,8 @@ static int run_class(qx_handle* h, int cls, int mode, const int2* d_q, long long
         TileArgs ta;
         ta.e = a;
         ta.rys = h->d_rys;
-        g_tile_launch[cls](ta, TK_PLAIN, mode, nq, h->work[cls].max_prims, s);
+        const ClassWork& w = h->work[cls];
+        g_tile_launch[cls](ta, TK_PLAIN, mode, nq, w.prims, w.max_prims, a.order ? w.prefix : nullptr, s);
     } else if (eng == ENG_COOP) {
         qx_launch_coop(g_coop_idx[cls], a, mode, s);
     } else if (eng == ENG_WARP || eng == ENG_WSPLIT) {
@@ -679,27 +688,30 @@ extern "C" int qx_initialize(int natom, const double* coords, int nshell, const 
         free_handle(h);
         return fail(QX_E_CUDA, "qx_initialize: Rys table not found on device %d", h->device);
     }
+    bool dropped = false;
+    for (int p = 0; p < np; ++p) dropped = dropped || (h->pairs[p].l1 <= 1 && h->pairs[p].nprim < h->nfull[p]);
+    std::vector<PairInfo> pairs(h->pairs);
+    const size_t nprims = prims.size();
+    if (dropped) {
+        prims.insert(prims.end(), prims_all.begin(), prims_all.end());
+        pairs.insert(pairs.end(), h->pairs.begin(), h->pairs.end());
+        for (int p = 0; p < np; ++p)
+            if (pairs[np + p].l1 <= 1) {
+                pairs[np + p].prim_off = all_off[p];
+                pairs[np + p].nprim = h->nfull[p];
+            }
+    }
     QX_ALLOC(h->d_prims, sizeof(PrimPair) * prims.size());
-    QX_ALLOC(h->d_pairs, sizeof(PairInfo) * np);
+    QX_ALLOC(h->d_pairs, sizeof(PairInfo) * pairs.size());
     QX_ALLOC(h->d_boys, sizeof(double) * boys.size());
     QX_ALLOC(h->d_err, sizeof(int));
     cudaMemcpy(h->d_prims, prims.data(), sizeof(PrimPair) * prims.size(), cudaMemcpyHostToDevice);
-    cudaMemcpy(h->d_pairs, h->pairs.data(), sizeof(PairInfo) * np, cudaMemcpyHostToDevice);
+    cudaMemcpy(h->d_pairs, pairs.data(), sizeof(PairInfo) * pairs.size(), cudaMemcpyHostToDevice);
     cudaMemcpy(h->d_boys, boys.data(), sizeof(double) * boys.size(), cudaMemcpyHostToDevice);
     cudaMemset(h->d_err, 0, sizeof(int));
-    bool dropped = false;
-    for (int p = 0; p < np; ++p) dropped = dropped || (h->pairs[p].l1 <= 1 && h->pairs[p].nprim < h->nfull[p]);
     if (dropped) {
-        std::vector<PairInfo> all(h->pairs);
-        for (int p = 0; p < np; ++p)
-            if (all[p].l1 <= 1) {
-                all[p].prim_off = all_off[p];
-                all[p].nprim = h->nfull[p];
-            }
-        QX_ALLOC(h->d_prims_all, sizeof(PrimPair) * prims_all.size());
-        QX_ALLOC(h->d_pairs_all, sizeof(PairInfo) * np);
-        cudaMemcpy(h->d_prims_all, prims_all.data(), sizeof(PrimPair) * prims_all.size(), cudaMemcpyHostToDevice);
-        cudaMemcpy(h->d_pairs_all, all.data(), sizeof(PairInfo) * np, cudaMemcpyHostToDevice);
+        h->d_prims_all = h->d_prims + nprims;
+        h->d_pairs_all = h->d_pairs + np;
     }
     // global accumulator scratch, sized for the largest launch that needs it
     {
@@ -1243,7 +1255,7 @@ static int run_tile_grad(qx_handle* h, int c, const double* D, double cj, double
     ta.cj = cj;
     ta.ck = ck;
     ta.grad = grad;
-    g_tile_launch[c](ta, TK_GRAD, 0, w.nq, w.max_prims, cs);
+    g_tile_launch[c](ta, TK_GRAD, 0, w.nq, w.prims, w.max_prims, w.d_order ? w.prefix : nullptr, cs);
     QX_CUDA(cudaGetLastError());
     return QX_OK;
 }
@@ -1251,12 +1263,13 @@ static int run_tile_grad(qx_handle* h, int c, const double* D, double cj, double
 // One class through its first-derivative engine on stream `cs`.
 static int run_deriv_class(qx_handle* h, int c, int mode, double* out, const double* D, double cj, double ck,
                            double* grad, int slice, cudaStream_t cs) {
-    if (h->deriv_eng[c] == ENG_RYS) {
+    const int eng = mode == QX_MODE_GRAD ? h->grad_eng[c] : h->deriv_eng[c];
+    if (eng == ENG_RYS) {
         if (mode == QX_MODE_GRAD) return run_tile_grad(h, c, D, cj, ck, grad, cs);
         if (mode == QX_MODE_DER_DENSE) return run_rys_derk(h, c, 1, out, nullptr, cs);
         return run_rys_derk(h, c, 1, out, &slice, cs);
     }
-    if (h->deriv_eng[c] == ENG_WARP) {
+    if (eng == ENG_WARP) {
         WarpArgs wa;
         wa.e = class_args(h, c, out);
         wa.wpq = h->wpq_deriv[c];
@@ -1282,14 +1295,14 @@ static int run_deriv_class(qx_handle* h, int c, int mode, double* out, const dou
             a.nq64 = w.nq64 - w.slice_q[sl];
             const int2* tk = w.d_dtasks + w.slice_t[sl];
             const long long nt = w.slice_t[sl + 1] - w.slice_t[sl];
-            if (h->deriv_eng[c] == ENG_WVRR) {
+            if (eng == ENG_WVRR) {
                 QX_CUDA(cudaMemsetAsync(w.d_dacc, 0, sizeof(double) * a.nq * nacc, cs));
                 EriArgs av = a;
                 av.prim_stage = h->prim_stage;
             av.wait_limit = h->wait_limit;
                 g_wvrr[c](av, tk, nt, qx_der_chunk(), w.d_dacc, (int)nacc, cs);
                 qx_launch_der_hrr(g_der_idx[c], a, mode, D, cj, ck, grad, slice, w.d_dacc, cs);
-            } else if (h->deriv_eng[c] == ENG_DSPLIT) {
+            } else if (eng == ENG_DSPLIT) {
                 const long long npad = (nacc + 15) / 16 * 16;  // the warp program's NITEM_PAD
                 QX_CUDA(cudaMemsetAsync(w.d_dacc, 0, sizeof(double) * a.nq * npad, cs));
                 EriArgs av = a;
@@ -1727,9 +1740,9 @@ extern "C" int qx_autotune(qx_handle* h, int what, void* stream) {
             if (g_der_idx[c] >= 0) cand.push_back({ENG_COOP, 0});
             cand.push_back({ENG_RYS, 0});
             float best = 1e30f;
-            TuneCfg bc{h->deriv_eng[c], h->wpq_deriv[c]};
+            TuneCfg bc{h->grad_eng[c], h->wpq_deriv[c]};
             for (const TuneCfg& t : cand) {
-                h->deriv_eng[c] = t.eng;
+                h->deriv_eng[c] = h->grad_eng[c] = t.eng;
                 if (t.eng == ENG_WARP) h->wpq_deriv[c] = t.param;
                 float ms = 0.f;
                 rc = time_config(s, e0, e1, &ms, [&] {
@@ -1741,7 +1754,7 @@ extern "C" int qx_autotune(qx_handle* h, int what, void* stream) {
                     bc = t;
                 }
             }
-            h->deriv_eng[c] = bc.eng;
+            h->deriv_eng[c] = h->grad_eng[c] = bc.eng;
             if (bc.eng == ENG_WARP) h->wpq_deriv[c] = bc.param;
         }
     }
@@ -1808,7 +1821,7 @@ extern "C" int qx_set_engine(qx_handle* h, int cls, int plain, int pparam, int d
         if (deriv == ENG_COOP) ok = g_der_idx[cls] >= 0;
         if (deriv == ENG_RYS) ok = dparam == 0 || dparam == 1;
         if (!ok) return no("derivative", deriv);
-        h->deriv_eng[cls] = deriv;
+        h->deriv_eng[cls] = h->grad_eng[cls] = deriv;
         if (deriv == ENG_WARP) h->wpq_deriv[cls] = dparam;
         if (deriv == ENG_RYS) h->rys_param[cls] = dparam;
     }
@@ -1862,8 +1875,8 @@ extern "C" int qx_engine_config(const qx_handle* h, int cls, int* cfg) {
     if (!h || !cfg || cls < 0 || cls >= QX_NCLS_ALL) return fail(QX_E_INVALID, "qx_engine_config: bad argument");
     cfg[0] = h->plain_eng[cls];
     cfg[1] = h->plain_eng[cls] == ENG_SL ? h->work[cls].log2g : (h->plain_eng[cls] == ENG_WARP ? h->wpq[cls] : 0);
-    cfg[2] = h->deriv_eng[cls];
-    cfg[3] = h->deriv_eng[cls] == ENG_WARP ? h->wpq_deriv[cls] : (h->deriv_eng[cls] == ENG_RYS ? h->rys_param[cls] : 0);
+    cfg[2] = h->grad_eng[cls];
+    cfg[3] = h->grad_eng[cls] == ENG_WARP ? h->wpq_deriv[cls] : (h->grad_eng[cls] == ENG_RYS ? h->rys_param[cls] : 0);
     return QX_OK;
 }
 

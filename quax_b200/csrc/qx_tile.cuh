@@ -125,6 +125,7 @@ enum { TK_PLAIN = 0, TK_GRAD = 1 };
 // ------------------------------------------------------------------ one class --
 constexpr int TILE_SMEM_TARGET = 72 * 1024;  // tables of a batch (bytes)
 constexpr int TILE_MAXW = 8;                 // warps per block
+constexpr int TILE_SEGS = 13;                // 4,096 primitives down to one
 
 template <int LA, int LB, int LC, int LD, int KIND>
 struct TileCls {
@@ -243,7 +244,12 @@ struct TileCls {
 struct TileArgs {
     EriArgs e;
     const double* rys = nullptr;
-    int parts = 1;  // blocks that share a quartet's primitives
+    // blocks: segment k holds the quartets [first[k], first[k + 1]) of the processing order,
+    // 2^k blocks each that share the quartet's primitives, from block start[k] on; the
+    // largest quartets have the highest k
+    int nseg = 1;
+    long long start[TILE_SEGS + 1] = {};
+    int first[TILE_SEGS + 1] = {};
     const double* D = nullptr;
     double cj = 0.0, ck = 0.0;
     double* grad = nullptr;  // 3N, atomic adds
@@ -729,7 +735,7 @@ struct TileBounds {
     static constexpr int REGS = REGS0 > 255 ? 255 : (REGS0 < 64 ? 64 : REGS0);
     static constexpr int BY_REGS = 65536 / (C::NT * REGS), BY_SMEM = 227 * 1024 / (C::SMEM + 1024);
     static constexpr int B0 = BY_REGS < BY_SMEM ? BY_REGS : BY_SMEM;
-    static constexpr int MINB = B0 < 1 ? 1 : (B0 > 8 ? 8 : B0);
+    static constexpr int MINB = B0 < 1 ? 1 : (B0 > 16 ? 16 : B0);
 };
 
 template <class C>
@@ -753,10 +759,13 @@ __global__ void __launch_bounds__(C::NT, TileBounds<C>::MINB) k_tile(TileArgs ta
     const typename Bra::Tab& tb = g_tile_tab<C::la, C::lb>;
     const typename Ket::Tab& tk = g_tile_tab<C::lc, C::ld>;
     const EriArgs& a = ta.e;
-    const long long n = a.n, qi = list_index(a, blockIdx.x);
+    int seg = ta.nseg - 1;  // block-uniform
+    while (seg > 0 && (long long)blockIdx.x >= ta.start[seg - 1]) --seg;
+    const int rel = (int)(blockIdx.x - ta.start[seg]), parts = 1 << seg;
+    const long long n = a.n, qi = list_index(a, ta.first[seg] + (rel >> seg));
     const int2 pq = a.quartets[qi];
     const int ntot = a.pairs[pq.x].nprim * a.pairs[pq.y].nprim;
-    const int part = blockIdx.y, stride = gridDim.y * C::PB;
+    const int part = rel & (parts - 1), stride = parts * C::PB;
     if (part * C::PB >= ntot) return;  // whole block
     if (tid < 24) {
         reinterpret_cast<int*>(&w.P)[tid] = reinterpret_cast<const int*>(a.pairs + pq.x)[tid];
@@ -886,7 +895,7 @@ __global__ void __launch_bounds__(C::NT, TileBounds<C>::MINB) k_tile(TileArgs ta
             jk_block<NA, NB, NC, ND>(a.out, a.out2, a.dens, n, w.P, w.Q, s12, s34, sPQ, tid, NT,
                                      [&](int o) { return out[o]; });
         } else {
-            const bool add = gridDim.y > 1;  // parts of a quartet meet in zeroed outputs
+            const bool add = parts > 1;  // parts of a quartet meet in zeroed outputs
             for (int o = tid; o < C::NCOMP; o += NT) {
                 const int ab = o / (NC * ND), cd = o - ab * (NC * ND);
                 const double v = tl_fwd_ket<C>(tk, coC, Hx, ab, cd);
@@ -904,20 +913,41 @@ __global__ void __launch_bounds__(C::NT, TileBounds<C>::MINB) k_tile(TileArgs ta
     }
 }
 
-// Blocks of a class: one per quartet; few quartets split their primitives until every SM
-// has several blocks (a quartet has 1 to 4,096 primitives, and the largest one would
-// otherwise be the launch's tail), never below two batches a block.
+// Blocks of a class.  A quartet has 1 to 4,096 primitives; with one block each the largest
+// ones were the tail of every launch (ten atoms, (22|21): the FP64 pipe 45% busy while
+// blocks ran, 26% over the launch).  A block takes at most `share` primitives: an eighth
+// of what each of the GPU's block slots gets in all, and two batches at least (gradient:
+// 48 primitives, about what its transfers of Gamma cost).  prefix[k]
+// counts the quartets with more than 2^k primitives in the processing order, which has
+// the largest first; without one (null: equal counts, or a list of its own) all quartets
+// are taken as the largest.
 template <class C>
-void launch_tile(TileArgs& ta, int mode, long long nq, int max_prims, cudaStream_t s) {
+void launch_tile(TileArgs& ta, int mode, long long nq, long long prims, int max_prims, const int* prefix, cudaStream_t s) {
     if (nq <= 0) return;
     auto k = k_tile<C>;
     if (C::SMEM > 40 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
-    const long long want = 148LL * TileBounds<C>::MINB * 6 / nq + 1;
-    const int batches = (max_prims + C::PB - 1) / C::PB;
-    const int parts = mode == MODE_SCHWARZ ? 1 : (int)std::min<long long>(want, std::max(1, batches / 2));
-    if (parts > 1 && !C::DER && mode == MODE_UNIQUE)
+    const long long share = std::max<long long>(C::DER ? std::max(2 * C::PB, 48) : 2 * C::PB,
+                                                prims / (148LL * TileBounds<C>::MINB * 8) + 1);
+    int low = 0;  // share rounded down to a power of two
+    while (low < TILE_SEGS - 1 && (2LL << low) <= share) ++low;
+    ta.nseg = 1;
+    if (mode != MODE_SCHWARZ)
+        while (ta.nseg < TILE_SEGS && (max_prims - 1) >> (low + ta.nseg - 1)) ++ta.nseg;
+    // segment j: more than 2^(low + j - 1) primitives (none has more than the last's)
+    long long blocks = 0;
+    int from = 0;
+    for (int j = ta.nseg - 1; j >= 0; --j) {
+        ta.first[j] = from;
+        ta.start[j] = blocks;
+        int to = (int)nq;
+        if (j > 0 && prefix) to = low + j - 1 < TILE_SEGS ? prefix[low + j - 1] : 0;
+        to = std::max(from, to);
+        blocks += (long long)(to - from) << j;
+        from = to;
+    }
+    if (ta.nseg > 1 && !C::DER && mode == MODE_UNIQUE)
         cudaMemsetAsync(ta.e.out + ta.e.base, 0, sizeof(double) * nq * C::NCOMP, s);
-    k<<<dim3((unsigned)nq, (unsigned)parts, C::NPASS), C::NT, C::SMEM, s>>>(ta, mode);
+    k<<<dim3((unsigned)blocks, 1, C::NPASS), C::NT, C::SMEM, s>>>(ta, mode);
 }
 #endif  // TILE_HOST
 
