@@ -1144,6 +1144,21 @@ def gen_rys(here, lmax_os):
         f.write("\n".join(H) + "\n")
 
 
+def gen_sljk(here, qc):
+    """One translation unit per straight-line class with its J/K launcher
+    qx_launch_sljk_<id>(args, stream)."""
+    for i, (a, b, c, d) in enumerate(qc):
+        if (a, b, c, d) in COOP_CLASSES:
+            continue
+        L = ["// Generated by quax_b200/csrc/gen_eri.py -- do not edit by hand.",
+             f"// J/K of the straight-line class ({a}{b}|{c}{d}).",
+             '#include "../qx_sljk.cuh"',
+             f"void qx_launch_sljk_{i}(const qx::EriArgs& a, cudaStream_t s) "
+             f"{{ qx::launch_sljk<{a}, {b}, {c}, {d}>(a, s); }}"]
+        with _Out(os.path.join(here, "gen", f"k_sljk_{i:02d}.cu")) as f:
+            f.write("\n".join(L) + "\n")
+
+
 def gen_tile(here):
     """One translation unit per class up to RYS_LMAX with the tile engine's launcher
     qx_launch_tile_<id>(args, kind, mode, nquartets, primitive quartets, the largest
@@ -1242,6 +1257,7 @@ def main():
         f.write(gen_coop_deriv(list(enumerate(qc))))
     gen_rys(here, lmax)
     gen_tile(here)
+    gen_sljk(here, qc)
 
 
 if __name__ == "__main__":

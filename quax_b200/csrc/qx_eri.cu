@@ -83,6 +83,11 @@ struct DeviceGuard {
 // Per-class launch table: straight-line kernels where generated, the
 // warp-cooperative engine for the large classes.
 static EriLaunch g_eri_launch[QX_NCLS_ALL];
+// J/K of the straight-line classes (gen/k_sljk_<id>.cu)
+#define QX_DECL_SLJK(id, a, b, c, d) void qx_launch_sljk_##id(const qx::EriArgs&, cudaStream_t);
+QX_FOR_EACH_SL_CLASS(QX_DECL_SLJK)
+#undef QX_DECL_SLJK
+static void (*g_sljk_launch[QX_NCLS_ALL])(const qx::EriArgs&, cudaStream_t);
 static long long g_class_scratch[QX_NCLS_ALL];
 static int g_class_nout[QX_NCLS_ALL];
 static const int g_class_coop[QX_NCLS_ALL] = QX_CLASS_COOP;
@@ -202,6 +207,7 @@ static bool init_class_tables() {
 #undef QX_TILE_ENTRY
 #define QX_SL_ENTRY(id, a, b, c, d)                            \
     g_eri_launch[id] = &qx_launch_eri_##id;                    \
+    g_sljk_launch[id] = &qx_launch_sljk_##id;                  \
     g_class_scratch[id] = qx::scratch_per_quartet<a, b, c, d>();
     QX_FOR_EACH_SL_CLASS(QX_SL_ENTRY)
     return true;
@@ -592,6 +598,8 @@ static int run_class(qx_handle* h, int cls, int mode, const int2* d_q, long long
             wa.acc_in = w.d_pacc;
         }
         g_warp_plain[cls](wa, mode, s);
+    } else if (mode == MODE_JK) {
+        g_sljk_launch[cls](a, s);
     } else {
         g_eri_launch[cls](a, mode, s);
     }

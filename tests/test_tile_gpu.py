@@ -47,3 +47,21 @@ def test_split_primitives(oracle_lib, ks):
     g = eng.grad_adjoint(Dg, 2.0, -1.0).cpu().numpy()
     gr = oracle_lib.grad_contract(ob, 1e-12, D, 2.0, -1.0)
     assert np.abs(g - gr).max() < 1e-9 * max(1.0, np.abs(gr).max())
+
+
+@pytest.mark.parametrize("lg", [0, 2, 5])
+def test_straight_line_jk(oracle_lib, lg):
+    """J/K of every class with a straight-line kernel, 2^lg lanes per quartet: accumulators
+    in registers and in shared memory, full and screened builds."""
+    b = synthetic_molecule(SyntheticSpec(natom=4, box=5.0, min_sep=1.2, kmax=2, exp_lo=0.1, exp_hi=50.0,
+                                         heavy_ls=(0, 0, 1, 1, 2), h_ls=(0, 0, 1)), 5)[1]
+    eng = EriEngine(b, 1e-12)
+    for c in eng.class_info():
+        if "%d%d%d%d" % c["l"] not in ("2121", "2211", "2221", "2222") and max(c["l"]) <= 2:
+            eng.set_engine(c["cls"], plain="sl", plain_param=lg)
+    G = oracle_lib.compute_2e_int(oracle_lib.OracleBasis(b), 1e-12)
+    D = _density(eng.nbf, 2)
+    for kw in ({}, {"screen": 1e-14}):
+        J, K = (x.cpu().numpy() for x in eng.jk(torch.from_numpy(D).cuda(), **kw))
+        assert np.abs(J - np.einsum("ijkl,kl->ij", G, D)).max() < 1e-10
+        assert np.abs(K - np.einsum("ikjl,kl->ij", G, D)).max() < 1e-10
