@@ -1090,8 +1090,11 @@ class _Out:
     unchanged, so a regeneration does not force the (slow) recompilation of
     every generated translation unit."""
 
+    written = set()  # paths of this run
+
     def __init__(self, path, mode="w"):
         self.path, self.parts = path, []
+        _Out.written.add(os.path.abspath(path))
 
     def __enter__(self):
         return self
@@ -1144,18 +1147,18 @@ def gen_rys(here, lmax_os):
         f.write("\n".join(H) + "\n")
 
 
-def gen_sljk(here, qc):
-    """One translation unit per straight-line class with its J/K launcher
-    qx_launch_sljk_<id>(args, stream)."""
+def gen_sl(here, qc):
+    """One translation unit per straight-line class with its launcher over segments of
+    equal lane count, qx_launch_sl_<id>(args, mode, stream)."""
     for i, (a, b, c, d) in enumerate(qc):
         if (a, b, c, d) in COOP_CLASSES:
             continue
         L = ["// Generated by quax_b200/csrc/gen_eri.py -- do not edit by hand.",
-             f"// J/K of the straight-line class ({a}{b}|{c}{d}).",
-             '#include "../qx_sljk.cuh"',
-             f"void qx_launch_sljk_{i}(const qx::EriArgs& a, cudaStream_t s) "
-             f"{{ qx::launch_sljk<{a}, {b}, {c}, {d}>(a, s); }}"]
-        with _Out(os.path.join(here, "gen", f"k_sljk_{i:02d}.cu")) as f:
+             f"// Straight-line kernels of class ({a}{b}|{c}{d}).",
+             '#include "../qx_sl.cuh"',
+             f"void qx_launch_sl_{i}(qx::SlArgs& a, int mode, cudaStream_t s) "
+             f"{{ qx::launch_sl<{a}, {b}, {c}, {d}>(a, mode, s); }}"]
+        with _Out(os.path.join(here, "gen", f"k_sl_{i:02d}.cu")) as f:
             f.write("\n".join(L) + "\n")
 
 
@@ -1257,7 +1260,12 @@ def main():
         f.write(gen_coop_deriv(list(enumerate(qc))))
     gen_rys(here, lmax)
     gen_tile(here)
-    gen_sljk(here, qc)
+    gen_sl(here, qc)
+    # translation units of an earlier generator would still be compiled
+    for name in os.listdir(os.path.join(here, "gen")):
+        path = os.path.abspath(os.path.join(here, "gen", name))
+        if name.endswith(".cu") and path not in _Out.written:
+            os.remove(path)
 
 
 if __name__ == "__main__":

@@ -7,8 +7,10 @@
 //   PairInfo[]  one record per shell pair (canonical order: higher AM first):
 //               A, AB = A - B, primitive range, basis-function offsets, atoms.
 //   int2[]      per angular-momentum class, the screened unique quartets
-//               (bra pair, ket pair), sorted by (bra nprim, ket nprim) so the
-//               primitive loops of a warp have equal trip counts.
+//               (bra pair, ket pair), sorted by the contracted primitive counts of
+//               bra and ket (the unique layout); kernels take them in the order of
+//               decreasing primitives left (EriArgs::order), so the primitive loops of
+//               a warp have equal trip counts.
 //   double[]    Boys table F_m(T_g), T_g = g/16, g = 0..BOYS_NG-1, m = 0..BOYS_NM-1,
 //               row-major [g][m] so the 8 Taylor coefficients of one T are adjacent.
 #pragma once

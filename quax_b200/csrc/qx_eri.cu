@@ -15,7 +15,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <chrono>
 #include <functional>
 #include <memory>
@@ -32,6 +31,7 @@
 #include "quax_b200.h"
 #include "qx_warp.cuh"
 #include "qx_rys.cuh"
+#include "qx_sl.cuh"
 #include "qx_tile.cuh"
 #include "qx_setup.h"
 #include "gen/warp_index.cuh"
@@ -82,12 +82,11 @@ struct DeviceGuard {
 
 // Per-class launch table: straight-line kernels where generated, the
 // warp-cooperative engine for the large classes.
-static EriLaunch g_eri_launch[QX_NCLS_ALL];
-// J/K of the straight-line classes (gen/k_sljk_<id>.cu)
-#define QX_DECL_SLJK(id, a, b, c, d) void qx_launch_sljk_##id(const qx::EriArgs&, cudaStream_t);
-QX_FOR_EACH_SL_CLASS(QX_DECL_SLJK)
-#undef QX_DECL_SLJK
-static void (*g_sljk_launch[QX_NCLS_ALL])(const qx::EriArgs&, cudaStream_t);
+// Straight-line classes over segments of equal lane count (gen/k_sl_<id>.cu)
+#define QX_DECL_SL(id, a, b, c, d) void qx_launch_sl_##id(qx::SlArgs&, int, cudaStream_t);
+QX_FOR_EACH_SL_CLASS(QX_DECL_SL)
+#undef QX_DECL_SL
+static void (*g_sl_launch[QX_NCLS_ALL])(qx::SlArgs&, int, cudaStream_t);
 static long long g_class_scratch[QX_NCLS_ALL];
 static int g_class_nout[QX_NCLS_ALL];
 static const int g_class_coop[QX_NCLS_ALL] = QX_CLASS_COOP;
@@ -172,7 +171,7 @@ static bool has_os(int c) { return c < QX_NUM_CLASSES; }  // generated Obara-Sai
 static bool init_class_tables() {
     static const int nout_os[QX_NUM_CLASSES] = QX_CLASS_NOUT;
     for (int c = 0; c < QX_NCLS_ALL; ++c) {
-        g_eri_launch[c] = nullptr;
+        g_sl_launch[c] = nullptr;
         g_class_scratch[c] = 0;
         g_coop_idx[c] = has_os(c) && g_class_coop[c] ? qx_coop_index(c) : -1;
         g_der_idx[c] = has_os(c) ? qx_der_index(c) : -1;
@@ -206,8 +205,7 @@ static bool init_class_tables() {
     QX_FOR_EACH_CLASS_ALL(QX_TILE_ENTRY)
 #undef QX_TILE_ENTRY
 #define QX_SL_ENTRY(id, a, b, c, d)                            \
-    g_eri_launch[id] = &qx_launch_eri_##id;                    \
-    g_sljk_launch[id] = &qx_launch_sljk_##id;                  \
+    g_sl_launch[id] = &qx_launch_sl_##id;                      \
     g_class_scratch[id] = qx::scratch_per_quartet<a, b, c, d>();
     QX_FOR_EACH_SL_CLASS(QX_SL_ENTRY)
     return true;
@@ -225,7 +223,8 @@ struct ClassWork {
     long long prims = 0;       // primitive quartets of the class
     int max_prims = 0;         // of its largest quartet
     int prefix[TILE_SEGS] = {};  // with an order: quartets with more than 2^k primitives
-    int log2g = 0;             // lanes per quartet = 2^log2g
+    int log2g = 0;             // lanes per quartet = 2^log2g, where the caller or the autotuner set them
+    bool sl_auto = true;       // straight-line lanes by the quartet's primitives (sl_segments)
     double* scratch = nullptr; // global accumulators (ACC_GLOBAL classes), owned
     // derivative split mode (largest classes): primitive-chunk tasks and the
     // per-quartet accumulator sums
@@ -344,32 +343,51 @@ static int build_orders(qx_handle* h, const int2* const* lists) {
     }
     std::unique_ptr<int[]> order(new int[(size_t)std::max(1LL, total)]);
     std::vector<char> uniform(QX_NCLS_ALL, 1);
-    std::atomic<int> next{0};
-    const int nt = total < 65536 ? 1 : (int)std::min(8u, std::max(1u, std::thread::hardware_concurrency()));
-    host_parallel(nt, [&](int) {
-        std::vector<int> pos(NB + 1);
-        std::vector<unsigned short> key;
-        for (int i; (i = next.fetch_add(1)) < QX_NCLS_ALL;) {
-            const int c = h->order[i];
-            const long long nq = h->work[c].nq;
-            if (!nq) continue;
-            const int2* L = lists[c];
-            std::fill(pos.begin(), pos.end(), 0);
-            key.resize((size_t)nq);
-            int most = 0;
-            for (long long q = 0; q < nq; ++q) {
-                const int np = h->pairs[L[q].x].nprim * h->pairs[L[q].y].nprim;
-                most = std::max(most, np);
-                key[q] = (unsigned short)(NB - std::min(np, NB));
-                ++pos[key[q] + 1];
-                if (key[q] != key[0]) uniform[c] = 0;
+    // a counting sort over host threads: thread t counts its contiguous range of every
+    // class, and after a scan in (key, thread) order writes it
+    const int nt = (int)std::max<long long>(1, std::min<long long>({16, (long long)std::thread::hardware_concurrency(),
+                                                                    total / 16384}));
+    std::vector<int> live;
+    for (int c = 0; c < QX_NCLS_ALL; ++c)
+        if (h->work[c].nq) live.push_back(c);
+    const size_t nl = live.size();
+    std::vector<std::vector<int>> hist(nt);
+    auto key = [&](const int2& q) { return NB - std::min(h->pairs[q.x].nprim * h->pairs[q.y].nprim, NB); };
+    host_parallel(nt, [&](int t) {
+        hist[t].assign(nl * NB, 0);
+        for (size_t k = 0; k < nl; ++k) {
+            const long long nq = h->work[live[k]].nq;
+            int* H = hist[t].data() + k * NB;
+            for (long long q = nq * t / nt; q < nq * (t + 1) / nt; ++q) ++H[key(lists[live[k]][q])];
+        }
+    });
+    host_parallel(nt, [&](int t) {
+        for (size_t k = t; k < nl; k += nt) {
+            ClassWork& w = h->work[live[k]];
+            int run = 0, above[NB + 1];
+            for (int b = 0; b < NB; ++b) {
+                above[b] = run;
+                for (int u = 0; u < nt; ++u) {
+                    int& x = hist[u][k * NB + b];
+                    const int v = x;
+                    x = run;
+                    run += v;
+                }
+                if (run != above[b] && run - above[b] != w.nq) uniform[live[k]] = 0;
+                if (above[b] == 0 && run) w.max_prims = NB - b;
             }
-            h->work[c].max_prims = most;
+            above[NB] = run;
+            for (int b = 0; b < TILE_SEGS; ++b) w.prefix[b] = above[NB - std::min(1 << b, NB)];
+        }
+    });
+    host_parallel(nt, [&](int t) {
+        for (size_t k = 0; k < nl; ++k) {
+            const int c = live[k];
             if (uniform[c]) continue;
-            for (int k = 0; k < NB; ++k) pos[k + 1] += pos[k];
-            for (int k = 0; k < TILE_SEGS; ++k) h->work[c].prefix[k] = pos[NB - std::min(1 << k, NB)];
+            const long long nq = h->work[c].nq;
+            int* H = hist[t].data() + k * NB;
             int* o = order.get() + off[c];
-            for (long long q = 0; q < nq; ++q) o[pos[key[q]]++] = (int)q;
+            for (long long q = nq * t / nt; q < nq * (t + 1) / nt; ++q) o[H[key(lists[c][q])]++] = (int)q;
         }
     });
     if (std::all_of(uniform.begin(), uniform.end(), [](char u) { return u != 0; })) return QX_OK;
@@ -535,6 +553,31 @@ static void free_handle(qx_handle* h) {
     delete h;
 }
 
+// Segments of a straight-line class: lanes per quartet so that a lane walks at most
+// `share` primitives -- what each of the GPU's resident threads (148 SMs, about 768) gets
+// of the class, at least 64, or 16 where there is not one primitive per thread and only
+// latency counts.  Smaller shares cost more in the transfer, which one lane of a group
+// runs, than they save in the tail, which other classes fill (ten atoms unique 4.21 ms at
+// 16, 3.94 at 64, 4.12 at 256; 12 atoms J/K 13.8, 13.2, 13.2; H2O 30 us at 16, 48 at 64).
+static void sl_segments(const ClassWork& w, SlArgs& sa) {
+    const long long threads = 148LL * 768;
+    const long long share = std::min(4096LL, w.prims < threads ? 16LL : std::max(64LL, w.prims / threads));
+    int low = 4;
+    while ((2LL << low) <= share) ++low;
+    int top = 0;  // lanes of the largest quartets
+    while (top < SL_SEGS - 1 && (w.max_prims - 1) >> (low + top)) ++top;
+    if (!w.d_order) {  // equal counts
+        sa.first[1] = (int)w.nq;
+        sa.lg[0] = top;
+        return;
+    }
+    sa.nseg = top + 1;
+    for (int k = 0; k <= top; ++k) {  // largest quartets, and most lanes, first
+        sa.lg[k] = top - k;
+        sa.first[k + 1] = k == top ? (int)w.nq : w.prefix[low + top - k - 1];
+    }
+}
+
 static int run_class(qx_handle* h, int cls, int mode, const int2* d_q, long long nq, double* out, long long n,
                      long long base, cudaStream_t s, int log2g = 0, double* scratch = nullptr, double* out2 = nullptr,
                      const double* dens = nullptr) {
@@ -598,10 +641,16 @@ static int run_class(qx_handle* h, int cls, int mode, const int2* d_q, long long
             wa.acc_in = w.d_pacc;
         }
         g_warp_plain[cls](wa, mode, s);
-    } else if (mode == MODE_JK) {
-        g_sljk_launch[cls](a, s);
     } else {
-        g_eri_launch[cls](a, mode, s);
+        SlArgs sa;
+        sa.e = a;
+        if (d_q == h->work[cls].d_q && h->work[cls].sl_auto) {
+            sl_segments(h->work[cls], sa);
+        } else {
+            sa.first[1] = (int)nq;
+            sa.lg[0] = log2g;
+        }
+        g_sl_launch[cls](sa, mode, s);
     }
     QX_CUDA(cudaGetLastError());
     return QX_OK;
@@ -1707,7 +1756,7 @@ extern "C" int qx_autotune(qx_handle* h, int what, void* stream) {
         if ((what & 1) && has_os(c)) {  // the f classes have one plain engine
             std::vector<TuneCfg> cand;
             if (!g_class_coop[c] && !g_class_scratch[c])
-                for (int lg = 0; lg <= 5; ++lg) cand.push_back({ENG_SL, lg});
+                for (int lg = -1; lg <= 5; ++lg) cand.push_back({ENG_SL, lg});  // -1: by primitives
             if (g_has_warp_plain[c]) {
                 cand.push_back({ENG_WARP, 1});
                 cand.push_back({ENG_WARP, 4});
@@ -1718,11 +1767,12 @@ extern "C" int qx_autotune(qx_handle* h, int what, void* stream) {
             cand.push_back({ENG_RYS, 0});
             const int keep_wpq = h->wpq[c], keep_lg = w.log2g;
             float best = 1e30f;
-            TuneCfg bc{h->plain_eng[c], h->plain_eng[c] == ENG_SL ? keep_lg : keep_wpq};
+            TuneCfg bc{h->plain_eng[c], h->plain_eng[c] == ENG_SL ? (w.sl_auto ? -1 : keep_lg) : keep_wpq};
             for (const TuneCfg& t : cand) {
                 h->plain_eng[c] = t.eng;
                 if (t.eng == ENG_WARP || t.eng == ENG_WSPLIT) h->wpq[c] = t.param;
-                const int lg = t.eng == ENG_SL ? t.param : 0;
+                const int lg = t.eng == ENG_SL ? std::max(0, t.param) : 0;
+                w.sl_auto = t.param < 0;
                 float ms = 0.f;
                 rc = time_config(s, e0, e1, &ms, [&] {
                     return run_class(h, c, MODE_UNIQUE, w.d_q, w.nq, d_out, 0, 0, s, lg, w.scratch);
@@ -1735,7 +1785,8 @@ extern "C" int qx_autotune(qx_handle* h, int what, void* stream) {
             }
             h->plain_eng[c] = bc.eng;
             h->wpq[c] = (bc.eng == ENG_WARP || bc.eng == ENG_WSPLIT) ? bc.param : keep_wpq;
-            w.log2g = bc.eng == ENG_SL ? bc.param : keep_lg;
+            w.sl_auto = bc.eng != ENG_SL || bc.param < 0;
+            w.log2g = w.sl_auto ? keep_lg : bc.param;
         }
         if ((what & 2) && !rc) {
             std::vector<TuneCfg> cand;
@@ -1817,7 +1868,10 @@ extern "C" int qx_set_engine(qx_handle* h, int cls, int plain, int pparam, int d
             if (rc) return rc;
         }
         h->plain_eng[cls] = plain;
-        if (plain == ENG_SL) w.log2g = pparam;
+        if (plain == ENG_SL) {
+            w.log2g = pparam;
+            w.sl_auto = false;
+        }
         if (plain == ENG_WARP) h->wpq[cls] = pparam;
         if (plain == ENG_WSPLIT) h->wpq[cls] = 1;
     }

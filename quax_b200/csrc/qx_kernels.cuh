@@ -110,20 +110,6 @@ __device__ __forceinline__ void jk_images(double* __restrict__ J, double* __rest
 }
 
 template <int NA, int NB, int NC, int ND>
-struct JKStore {
-    double* __restrict__ J;
-    double* __restrict__ K;
-    const double* __restrict__ D;
-    long long n;
-    int bf1, bf2, bf3, bf4;
-    bool s12, s34, sPQ;
-    __device__ __forceinline__ void operator()(int k, double v) {
-        const int id = k % ND, ic = (k / ND) % NC, ib = (k / (ND * NC)) % NB, ia = k / (ND * NC * NB);
-        jk_images(J, K, D, n, bf1 + ia, bf2 + ib, bf3 + ic, bf4 + id, s12, s34, sPQ, v);
-    }
-};
-
-template <int NA, int NB, int NC, int ND>
 struct UniqueStore {
     double* out;
     long long base, nq, qi;
@@ -204,10 +190,6 @@ __device__ __noinline__ void finish_quartet(const EriArgs& a, const PairInfo& P,
         SchwarzStore<NA, NB, NC, ND> st;
         C::hrr(acc, st, P.ABx, P.ABy, P.ABz, Q.ABx, Q.ABy, Q.ABz);
         a.out[pq.x] = st.mx;
-    } else if constexpr (MODE == MODE_JK) {
-        JKStore<NA, NB, NC, ND> st{a.out, a.out2, a.dens, a.n, P.bf1, P.bf2, Q.bf1, Q.bf2,
-                                   P.s1 != P.s2, Q.s1 != Q.s2, pq.x != pq.y};
-        C::hrr(acc, st, P.ABx, P.ABy, P.ABz, Q.ABx, Q.ABy, Q.ABz);
     } else {
         DenseStore<NA, NB, NC, ND> st{a.out, a.n, P.bf1, P.bf2, Q.bf1, Q.bf2, P.s1 != P.s2, Q.s1 != Q.s2, pq.x != pq.y};
         C::hrr(acc, st, P.ABx, P.ABy, P.ABz, Q.ABx, Q.ABy, Q.ABz);
@@ -221,13 +203,12 @@ __global__ void __launch_bounds__(AccPolicy<EriCls<LA, LB, LC, LD>::NACC>::bs) k
     const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long qi = gt >> a.log2g;
     const int sub = (int)(gt & ((1 << a.log2g) - 1));
-    bool active = qi < a.nq;
+    const bool active = qi < a.nq;
     if (active) qi = list_index(a, qi);
     // every lane stays to the end: the group reduction shuffles over the full warp
     const int2 pq = active ? a.quartets[qi] : make_int2(0, 0);
     const PairInfo P = a.pairs[pq.x];
     const PairInfo Q = a.pairs[pq.y];
-    if (MODE == MODE_JK && active && jk_screened(a, pq, P, Q)) active = false;  // group-uniform
     if constexpr (Pol::kind == ACC_REG) {
         RegAcc<C::NACC> acc;
         contract_quartet<C>(a, P, Q, acc, sub, active);
@@ -257,10 +238,6 @@ void launch_eri(const EriArgs& a, int mode, cudaStream_t s) {
         k<<<(unsigned)nb, bs, Pol::smem, s>>>(a);
     } else if (mode == MODE_UNIQUE) {
         auto k = k_eri<LA, LB, LC, LD, MODE_UNIQUE>;
-        if (Pol::smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, Pol::smem);
-        k<<<(unsigned)nb, bs, Pol::smem, s>>>(a);
-    } else if (mode == MODE_JK) {
-        auto k = k_eri<LA, LB, LC, LD, MODE_JK>;
         if (Pol::smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, Pol::smem);
         k<<<(unsigned)nb, bs, Pol::smem, s>>>(a);
     } else if constexpr (LA == LC && LB == LD) {

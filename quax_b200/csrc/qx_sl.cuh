@@ -1,16 +1,36 @@
-// qx_sljk.cuh -- direct J/K of the straight-line classes (2^log2g lanes per quartet).
+// qx_sl.cuh -- the straight-line class kernels over a handle's quartet lists: 2^lg lanes
+// per quartet, lg by the quartet's primitives.
 //
-// The quartet's block regroups into the six contractions of qx_jk.cuh inside the lane
+// A lane that walks a quartet of 4,096 primitives takes a hundred times as long as its
+// average neighbour, and with one lane count per launch such quartets were its tail: ten
+// atoms, (ds|ps): FP64 pipe 52% busy while blocks ran, 20% over the launch.  The
+// processing order has the largest quartets first, so a launch is cut into segments of
+// equal lane count that keep a lane's share of primitives below a bound (SlArgs).
+//
+// J/K: the quartet's block regroups into the six contractions of qx_jk.cuh inside the lane
 // that owns it: every integral, as the transfer forms it, is folded into the sums over
 // its quartet's J and K entries, which then take one atomic per entry and image instead
 // of one per integral and image -- 24 instead of 48 for (ps|ss), 114 instead of 864 for
-// (dp|ps).  Those atomics bound the straight-line classes; now their recurrences do, and
-// summing the entries that neighbouring lanes share (J_AB, K_AC) over the warp first
-// changed nothing.  12 atoms (n = 160): J/K 18.4 -> 15.1 ms.
+// (dp|ps).  Summing the entries that neighbouring lanes share (J_AB, K_AC) over the warp
+// first changed nothing: the recurrences bound these kernels, not the atomics.
+// Ten atoms unique 4.18 -> 3.94 ms, dense (8 atoms) 2.05 -> 1.98 ms, J/K of 12 atoms
+// 18.4 ms integral by integral -> 15.4 by blocks -> 13.2 by segments.
 #pragma once
 #include "qx_kernels.cuh"
 
 namespace qx {
+
+constexpr int SL_SEGS = 6;  // 1 to 32 lanes
+
+// Segment k holds the quartets [first[k], first[k + 1]) of the processing order, 2^lg[k]
+// lanes each, from block start[k] on.
+struct SlArgs {
+    EriArgs e;
+    int nseg = 1;
+    long long start[SL_SEGS] = {};
+    int first[SL_SEGS + 1] = {};
+    int lg[SL_SEGS] = {};
+};
 
 template <int NA, int NB, int NC, int ND>
 struct SlJkSums {
@@ -81,45 +101,61 @@ __device__ __noinline__ void finish_jk(const EriArgs& a, const PairInfo& P, cons
     if (s12 && s34) sl_jk_add<NB, ND>(a.out2, n, B, Dd, sPQ, 1.0, st.kBD);
 }
 
-template <int LA, int LB, int LC, int LD>
-__global__ void __launch_bounds__(AccPolicy<EriCls<LA, LB, LC, LD>::NACC>::bs) k_sljk(EriArgs a) {
+template <int LA, int LB, int LC, int LD, int MODE>
+__global__ void __launch_bounds__(AccPolicy<EriCls<LA, LB, LC, LD>::NACC>::bs) k_sl(SlArgs sa) {
     using C = EriCls<LA, LB, LC, LD>;
     using Pol = AccPolicy<C::NACC>;
-    const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    long long qi = gt >> a.log2g;
+    static_assert(Pol::kind != ACC_GLOBAL, "straight-line classes keep their accumulators on the SM");
+    int seg = sa.nseg - 1;  // block-uniform
+    while (seg > 0 && (long long)blockIdx.x < sa.start[seg]) --seg;
+    EriArgs a = sa.e;
+    a.log2g = sa.lg[seg];
+    const long long gt = ((long long)blockIdx.x - sa.start[seg]) * Pol::bs + threadIdx.x;
+    long long qi = sa.first[seg] + (gt >> a.log2g);
     const int sub = (int)(gt & ((1 << a.log2g) - 1));
-    bool active = qi < a.nq;
+    bool active = qi < sa.first[seg + 1];
     if (active) qi = list_index(a, qi);
     // every lane stays to the end: the group reduction shuffles over the full warp
     const int2 pq = active ? a.quartets[qi] : make_int2(0, 0);
     const PairInfo P = a.pairs[pq.x];
     const PairInfo Q = a.pairs[pq.y];
-    if (active && jk_screened(a, pq, P, Q)) active = false;  // group-uniform
+    if (MODE == MODE_JK && active && jk_screened(a, pq, P, Q)) active = false;  // group-uniform
     auto go = [&](auto& acc) {
         contract_quartet<C>(a, P, Q, acc, sub, active);
-        if (active && sub == 0) finish_jk<C, LA, LB, LC, LD>(a, P, Q, pq, acc);
+        if (!active || sub) return;
+        if constexpr (MODE == MODE_JK) finish_jk<C, LA, LB, LC, LD>(a, P, Q, pq, acc);
+        else finish_quartet<C, LA, LB, LC, LD, MODE>(a, P, Q, pq, qi, acc);
     };
     if constexpr (Pol::kind == ACC_REG) {
         RegAcc<C::NACC> acc;
         go(acc);
-    } else if constexpr (Pol::kind == ACC_SMEM) {
+    } else {
         extern __shared__ double smem_acc[];
         StridedAcc acc{smem_acc + threadIdx.x, Pol::bs};
-        go(acc);
-    } else {
-        StridedAcc acc{a.scratch + gt, (long long)gridDim.x * blockDim.x};
         go(acc);
     }
 }
 
-template <int LA, int LB, int LC, int LD>
-void launch_sljk(const EriArgs& a, cudaStream_t s) {
+template <int LA, int LB, int LC, int LD, int MODE>
+void launch_sl_mode(SlArgs& sa, cudaStream_t s) {
     using Pol = AccPolicy<EriCls<LA, LB, LC, LD>::NACC>;
-    const long long nb = ((a.nq << a.log2g) + Pol::bs - 1) / Pol::bs;
-    if (nb == 0) return;
-    auto k = k_sljk<LA, LB, LC, LD>;
+    long long blocks = 0;
+    for (int k = 0; k < sa.nseg; ++k) {
+        sa.start[k] = blocks;
+        blocks += (((long long)(sa.first[k + 1] - sa.first[k]) << sa.lg[k]) + Pol::bs - 1) / Pol::bs;
+    }
+    if (blocks == 0) return;
+    auto k = k_sl<LA, LB, LC, LD, MODE>;
     if (Pol::smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, Pol::smem);
-    k<<<(unsigned)nb, Pol::bs, Pol::smem, s>>>(a);
+    k<<<(unsigned)blocks, Pol::bs, Pol::smem, s>>>(sa);
+}
+
+template <int LA, int LB, int LC, int LD>
+void launch_sl(SlArgs& sa, int mode, cudaStream_t s) {
+    if (mode == MODE_DENSE) return launch_sl_mode<LA, LB, LC, LD, MODE_DENSE>(sa, s);
+    if (mode == MODE_UNIQUE) return launch_sl_mode<LA, LB, LC, LD, MODE_UNIQUE>(sa, s);
+    if (mode == MODE_JK) return launch_sl_mode<LA, LB, LC, LD, MODE_JK>(sa, s);
+    if constexpr (LA == LC && LB == LD) launch_sl_mode<LA, LB, LC, LD, MODE_SCHWARZ>(sa, s);
 }
 
 }  // namespace qx

@@ -49,6 +49,32 @@ def test_split_primitives(oracle_lib, ks):
     assert np.abs(g - gr).max() < 1e-9 * max(1.0, np.abs(gr).max())
 
 
+@pytest.mark.parametrize("ks", [(8,), (1, 8), (1, 3, 8)])
+def test_straight_line_segments(oracle_lib, ks):
+    """The default lanes per quartet, by its primitives: 1 to 4,096 per quartet, equal
+    counts (one segment, no processing order) and mixed ones, in every output mode."""
+    rng = np.random.default_rng(11)
+    shells = []
+    for a, x in enumerate(([0.0, 0.0, 0.0], [0.4, -1.1, 1.9], [1.7, 1.2, -0.6])):
+        for i, l in enumerate((0, 0, 1, 2) if a else (0, 1, 1)):
+            k = ks[(i + a) % len(ks)]
+            e = np.sort(np.exp(rng.uniform(np.log(0.2), np.log(20.0), size=k)))[::-1].copy()
+            shells.append(Shell(l, e, rng.uniform(0.2, 1.0, size=k), np.array(x), a))
+    b = Basis(shells, 3)
+    ob = oracle_lib.OracleBasis(b)
+    eng = EriEngine(b, 1e-12)
+    assert sum(v[0] == "sl" for v in eng.engine_config().values()) >= 8
+    G = oracle_lib.compute_2e_int(ob, 1e-12)
+    assert np.abs(eng.eri().cpu().numpy() - G).max() < 1e-12
+    D = _density(eng.nbf, 4)
+    J, K = (x.cpu().numpy() for x in eng.jk(torch.from_numpy(D).cuda()))
+    assert np.abs(J - np.einsum("ijkl,kl->ij", G, D)).max() < 1e-10
+    assert np.abs(K - np.einsum("ikjl,kl->ij", G, D)).max() < 1e-10
+    for cls, (sh, blk) in eng.unique_blocks().items():
+        for s, v in zip(sh[:40], blk[:40].cpu().numpy()):
+            assert np.abs(v - oracle_lib.shell_quartet(ob, *map(int, s)).reshape(-1)).max() < 1e-12, cls
+
+
 @pytest.mark.parametrize("lg", [0, 2, 5])
 def test_straight_line_jk(oracle_lib, lg):
     """J/K of every class with a straight-line kernel, 2^lg lanes per quartet: accumulators
