@@ -1798,10 +1798,12 @@ extern "C" int qx_autotune(qx_handle* h, int what, void* stream) {
             if (g_has_dsplit[c]) cand.push_back({ENG_DSPLIT, 0});
             if (g_der_idx[c] >= 0) cand.push_back({ENG_COOP, 0});
             cand.push_back({ENG_RYS, 0});
-            float best = 1e30f;
-            TuneCfg bc{h->grad_eng[c], h->wpq_deriv[c]};
+            // the tile gradient says nothing about the Rys engine's tensors, so those keep
+            // the fastest of the class's other engines
+            float best = 1e30f, best_t = 1e30f;
+            TuneCfg bc{h->grad_eng[c], h->wpq_deriv[c]}, bt{h->deriv_eng[c], h->wpq_deriv[c]};
             for (const TuneCfg& t : cand) {
-                h->deriv_eng[c] = h->grad_eng[c] = t.eng;
+                h->grad_eng[c] = t.eng;
                 if (t.eng == ENG_WARP) h->wpq_deriv[c] = t.param;
                 float ms = 0.f;
                 rc = time_config(s, e0, e1, &ms, [&] {
@@ -1812,9 +1814,14 @@ extern "C" int qx_autotune(qx_handle* h, int what, void* stream) {
                     best = ms;
                     bc = t;
                 }
+                if (t.eng != ENG_RYS && ms < best_t) {
+                    best_t = ms;
+                    bt = t;
+                }
             }
-            h->deriv_eng[c] = h->grad_eng[c] = bc.eng;
-            if (bc.eng == ENG_WARP) h->wpq_deriv[c] = bc.param;
+            h->grad_eng[c] = bc.eng;
+            h->deriv_eng[c] = bt.eng;
+            if (bt.eng == ENG_WARP) h->wpq_deriv[c] = bt.param;  // bc's too, if it is a warp engine
         }
     }
     if (!rc) {
