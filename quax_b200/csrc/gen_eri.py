@@ -1172,7 +1172,7 @@ def gen_tile(here):
              f"// Tile-engine launchers of class ({a}{b}|{c}{d}).",
              '#include "../qx_tile.cuh"',
              f"void qx_launch_tile_{i:02d}(qx::TileArgs& ta, int kind, int mode, long long nq, long long prims, "
-             "int max_prims, const int* prefix, cudaStream_t s) {"]
+             "long long max_prims, const long long* prefix, cudaStream_t s) {"]
         for k in ("TK_PLAIN", "TK_GRAD"):
             L.append(f"    if (kind == qx::{k}) return qx::launch_tile<qx::TileCls<{a}, {b}, {c}, {d}, qx::{k}>>"
                      "(ta, mode, nq, prims, max_prims, prefix, s);")

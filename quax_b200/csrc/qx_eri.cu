@@ -33,6 +33,7 @@
 #include "qx_rys.cuh"
 #include "qx_sl.cuh"
 #include "qx_tile.cuh"
+#include "qx_segments.h"
 #include "qx_setup.h"
 #include "gen/warp_index.cuh"
 #include "gen/rys_index.cuh"
@@ -107,10 +108,10 @@ QX_FOR_EACH_CLASS_ALL(QX_DECL_RYS)
 #undef QX_DECL_RYS
 static RysLaunch g_rys_launch[QX_NCLS_ALL];
 // Tile-engine launchers, one per class (gen/k_tile_<id>.cu).
-typedef void (*TileLaunch)(qx::TileArgs&, int kind, int mode, long long nq, long long prims, int max_prims,
-                           const int* prefix, cudaStream_t);
-#define QX_DECL_TILE(id, a, b, c, d) \
-    void qx_launch_tile_##id(qx::TileArgs&, int, int, long long, long long, int, const int*, cudaStream_t);
+typedef void (*TileLaunch)(qx::TileArgs&, int kind, int mode, long long nq, long long prims, long long max_prims,
+                           const long long* prefix, cudaStream_t);
+#define QX_DECL_TILE(id, a, b, c, d)                                                                              \
+    void qx_launch_tile_##id(qx::TileArgs&, int, int, long long, long long, long long, const long long*, cudaStream_t);
 QX_FOR_EACH_CLASS_ALL(QX_DECL_TILE)
 #undef QX_DECL_TILE
 static TileLaunch g_tile_launch[QX_NCLS_ALL];
@@ -221,8 +222,9 @@ struct ClassWork {
     long long nq_full = 0;
     long long unique_base = 0;
     long long prims = 0;       // primitive quartets of the class
-    int max_prims = 0;         // of its largest quartet
-    int prefix[TILE_SEGS] = {};  // with an order: quartets with more than 2^k primitives
+    long long max_prims = 0;   // of its largest quartet
+    bool uniform = true;       // quartets of equal primitive counts
+    long long prefix[SEG_POW] = {};  // with an order: quartets with more than 2^k primitives
     int log2g = 0;             // lanes per quartet = 2^log2g, where the caller or the autotuner set them
     bool sl_auto = true;       // straight-line lanes by the quartet's primitives (sl_segments)
     double* scratch = nullptr; // global accumulators (ACC_GLOBAL classes), owned
@@ -329,76 +331,98 @@ static void host_parallel(int nt, F&& f) {
 // largest first, stable.  The list itself keeps the order of the contracted primitive
 // counts (the unique layout); once negligible primitive pairs are dropped, neighbours
 // there differ several-fold in work, and a straight-line kernel's warp takes as long as
-// its longest lane.  A class of equal counts needs none.
+// its longest lane.  A class of equal counts needs none, and one of more than 2^31 - 1
+// quartets, whose positions the order's entries do not hold, runs in list order.
 static int build_orders(qx_handle* h, const int2* const* lists) {
     cudaFree(h->d_orders);
     h->d_orders = nullptr;
-    constexpr int NB = 4096;
-    long long total = 0;
+    // keys up to the largest quartet of the handle
+    int pmax = 1;
+    for (const auto& p : h->pairs) pmax = std::max(pmax, p.nprim);
+    const int NB = seg_key((long long)pmax * pmax) + 1;
+    long long total = 0, work = 0;
     std::vector<long long> off(QX_NCLS_ALL, 0);
+    std::vector<int> live;
     for (int c = 0; c < QX_NCLS_ALL; ++c) {
-        h->work[c].d_order = nullptr;
+        ClassWork& w = h->work[c];
+        w.d_order = nullptr;
         off[c] = total;
-        total += h->work[c].nq;
+        if (!w.nq) continue;
+        live.push_back(c);
+        work += w.nq;
+        if (w.nq <= 0x7fffffffLL) total += w.nq;
     }
     std::unique_ptr<int[]> order(new int[(size_t)std::max(1LL, total)]);
-    std::vector<char> uniform(QX_NCLS_ALL, 1);
     // a counting sort over host threads: thread t counts its contiguous range of every
     // class, and after a scan in (key, thread) order writes it
     const int nt = (int)std::max<long long>(1, std::min<long long>({16, (long long)std::thread::hardware_concurrency(),
-                                                                    total / 16384}));
-    std::vector<int> live;
-    for (int c = 0; c < QX_NCLS_ALL; ++c)
-        if (h->work[c].nq) live.push_back(c);
+                                                                    work / 16384}));
     const size_t nl = live.size();
-    std::vector<std::vector<int>> hist(nt);
-    auto key = [&](const int2& q) { return NB - std::min(h->pairs[q.x].nprim * h->pairs[q.y].nprim, NB); };
+    std::vector<std::vector<long long>> hist(nt);
+    auto prims = [&](const int2& q) { return (long long)h->pairs[q.x].nprim * h->pairs[q.y].nprim; };
+    auto key = [&](const int2& q) { return NB - 1 - seg_key(prims(q)); };  // largest first
     host_parallel(nt, [&](int t) {
         hist[t].assign(nl * NB, 0);
         for (size_t k = 0; k < nl; ++k) {
             const long long nq = h->work[live[k]].nq;
-            int* H = hist[t].data() + k * NB;
+            long long* H = hist[t].data() + k * NB;
             for (long long q = nq * t / nt; q < nq * (t + 1) / nt; ++q) ++H[key(lists[live[k]][q])];
         }
     });
     host_parallel(nt, [&](int t) {
+        std::vector<long long> sum(NB);
         for (size_t k = t; k < nl; k += nt) {
             ClassWork& w = h->work[live[k]];
-            int run = 0, above[NB + 1];
+            long long run = 0;
+            int used = 0;
             for (int b = 0; b < NB; ++b) {
-                above[b] = run;
+                const long long before = run;
                 for (int u = 0; u < nt; ++u) {
-                    int& x = hist[u][k * NB + b];
-                    const int v = x;
+                    long long& x = hist[u][k * NB + b];
+                    const long long v = x;
                     x = run;
                     run += v;
                 }
-                if (run != above[b] && run - above[b] != w.nq) uniform[live[k]] = 0;
-                if (above[b] == 0 && run) w.max_prims = NB - b;
+                sum[NB - 1 - b] = run - before;
+                used += run != before;
             }
-            above[NB] = run;
-            for (int b = 0; b < TILE_SEGS; ++b) w.prefix[b] = above[NB - std::min(1 << b, NB)];
+            w.uniform = used == 1;
+            seg_prefix(sum.data(), NB, w.prefix);
         }
     });
+    std::vector<long long> top((size_t)nt * nl, 0);
     host_parallel(nt, [&](int t) {
         for (size_t k = 0; k < nl; ++k) {
             const int c = live[k];
-            if (uniform[c]) continue;
-            const long long nq = h->work[c].nq;
-            int* H = hist[t].data() + k * NB;
+            const ClassWork& w = h->work[c];
+            const long long nq = w.nq;
+            const bool sort = !w.uniform && nq <= 0x7fffffffLL;
+            long long* H = hist[t].data() + k * NB;
             int* o = order.get() + off[c];
-            for (long long q = nq * t / nt; q < nq * (t + 1) / nt; ++q) o[H[key(lists[c][q])]++] = (int)q;
+            long long mx = 0;
+            for (long long q = nq * t / nt; q < nq * (t + 1) / nt; ++q) {
+                mx = std::max(mx, prims(lists[c][q]));
+                if (sort) o[H[key(lists[c][q])]++] = (int)q;
+            }
+            top[(size_t)t * nl + k] = mx;
         }
     });
-    if (std::all_of(uniform.begin(), uniform.end(), [](char u) { return u != 0; })) return QX_OK;
+    bool any = false;
+    for (size_t k = 0; k < nl; ++k) {
+        ClassWork& w = h->work[live[k]];
+        w.max_prims = 0;
+        for (int t = 0; t < nt; ++t) w.max_prims = std::max(w.max_prims, top[(size_t)t * nl + k]);
+        any = any || (!w.uniform && w.nq <= 0x7fffffffLL);
+    }
+    if (!any) return QX_OK;
     if (cudaMalloc((void**)&h->d_orders, sizeof(int) * total) != cudaSuccess) {
         cudaGetLastError();
         h->d_orders = nullptr;
         return fail(QX_E_NOMEM, "processing order of %lld quartets", total);
     }
     QX_CUDA(cudaMemcpy(h->d_orders, order.get(), sizeof(int) * total, cudaMemcpyHostToDevice));
-    for (int c = 0; c < QX_NCLS_ALL; ++c)
-        if (!uniform[c]) h->work[c].d_order = h->d_orders + off[c];
+    for (int c : live)
+        if (!h->work[c].uniform && h->work[c].nq <= 0x7fffffffLL) h->work[c].d_order = h->d_orders + off[c];
     return QX_OK;
 }
 
@@ -553,31 +577,6 @@ static void free_handle(qx_handle* h) {
     delete h;
 }
 
-// Segments of a straight-line class: lanes per quartet so that a lane walks at most
-// `share` primitives -- what each of the GPU's resident threads (148 SMs, about 768) gets
-// of the class, at least 64, or 16 where there is not one primitive per thread and only
-// latency counts.  Smaller shares cost more in the transfer, which one lane of a group
-// runs, than they save in the tail, which other classes fill (ten atoms unique 4.21 ms at
-// 16, 3.94 at 64, 4.12 at 256; 12 atoms J/K 13.8, 13.2, 13.2; H2O 30 us at 16, 48 at 64).
-static void sl_segments(const ClassWork& w, SlArgs& sa) {
-    const long long threads = 148LL * 768;
-    const long long share = std::min(4096LL, w.prims < threads ? 16LL : std::max(64LL, w.prims / threads));
-    int low = 4;
-    while ((2LL << low) <= share) ++low;
-    int top = 0;  // lanes of the largest quartets
-    while (top < SL_SEGS - 1 && (w.max_prims - 1) >> (low + top)) ++top;
-    if (!w.d_order) {  // equal counts
-        sa.first[1] = (int)w.nq;
-        sa.lg[0] = top;
-        return;
-    }
-    sa.nseg = top + 1;
-    for (int k = 0; k <= top; ++k) {  // largest quartets, and most lanes, first
-        sa.lg[k] = top - k;
-        sa.first[k + 1] = k == top ? (int)w.nq : w.prefix[low + top - k - 1];
-    }
-}
-
 static int run_class(qx_handle* h, int cls, int mode, const int2* d_q, long long nq, double* out, long long n,
                      long long base, cudaStream_t s, int log2g = 0, double* scratch = nullptr, double* out2 = nullptr,
                      const double* dens = nullptr) {
@@ -645,9 +644,11 @@ static int run_class(qx_handle* h, int cls, int mode, const int2* d_q, long long
         SlArgs sa;
         sa.e = a;
         if (d_q == h->work[cls].d_q && h->work[cls].sl_auto) {
-            sl_segments(h->work[cls], sa);
+            const ClassWork& w = h->work[cls];
+            sa.nseg = sl_segments(w.nq, w.prims, w.max_prims, w.d_order ? w.prefix : nullptr,
+                                  w.uniform ? -1 : choose_log2g(w.nq, w.prims), sa.first, sa.lg);
         } else {
-            sa.first[1] = (int)nq;
+            sa.first[1] = nq;
             sa.lg[0] = log2g;
         }
         g_sl_launch[cls](sa, mode, s);
@@ -1258,8 +1259,8 @@ static int rys_unsupported(int c, const char* what) {
 // Work items that share a quartet's primitives in the Rys kernels: a team walks its
 // primitives one after another (up to 4,096 of them), so few quartets would leave most
 // of the GPU idle behind the largest one.  The outputs are sums of atomics either way.
-static int rys_parts(long long items, int max_prims) {
-    return (int)std::min<long long>(148LL * 32 / items + 1, std::max(1, max_prims / 4));
+static int rys_parts(long long items, long long max_prims) {
+    return (int)std::min(148LL * 32 / items + 1, std::max(1LL, max_prims / 4));
 }
 
 // Derivative tensor of order k (1..4) of one class through the Rys engine:

@@ -17,10 +17,9 @@
 // 18.4 ms integral by integral -> 15.4 by blocks -> 13.2 by segments.
 #pragma once
 #include "qx_kernels.cuh"
+#include "qx_segments.h"
 
 namespace qx {
-
-constexpr int SL_SEGS = 6;  // 1 to 32 lanes
 
 // Segment k holds the quartets [first[k], first[k + 1]) of the processing order, 2^lg[k]
 // lanes each, from block start[k] on.
@@ -28,7 +27,7 @@ struct SlArgs {
     EriArgs e;
     int nseg = 1;
     long long start[SL_SEGS] = {};
-    int first[SL_SEGS + 1] = {};
+    long long first[SL_SEGS + 1] = {};
     int lg[SL_SEGS] = {};
 };
 
@@ -142,7 +141,7 @@ void launch_sl_mode(SlArgs& sa, cudaStream_t s) {
     long long blocks = 0;
     for (int k = 0; k < sa.nseg; ++k) {
         sa.start[k] = blocks;
-        blocks += (((long long)(sa.first[k + 1] - sa.first[k]) << sa.lg[k]) + Pol::bs - 1) / Pol::bs;
+        blocks += (((sa.first[k + 1] - sa.first[k]) << sa.lg[k]) + Pol::bs - 1) / Pol::bs;
     }
     if (blocks == 0) return;
     auto k = k_sl<LA, LB, LC, LD, MODE>;

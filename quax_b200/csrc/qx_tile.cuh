@@ -39,6 +39,7 @@
 
 #include "qx_jk.cuh"
 #include "qx_rys.cuh"
+#include "qx_segments.h"
 
 namespace qx {
 
@@ -125,7 +126,6 @@ enum { TK_PLAIN = 0, TK_GRAD = 1 };
 // ------------------------------------------------------------------ one class --
 constexpr int TILE_SMEM_TARGET = 72 * 1024;  // tables of a batch (bytes)
 constexpr int TILE_MAXW = 8;                 // warps per block
-constexpr int TILE_SEGS = 13;                // 4,096 primitives down to one
 
 template <int LA, int LB, int LC, int LD, int KIND>
 struct TileCls {
@@ -244,12 +244,12 @@ struct TileCls {
 struct TileArgs {
     EriArgs e;
     const double* rys = nullptr;
-    // blocks: segment k holds the quartets [first[k], first[k + 1]) of the processing order,
-    // 2^k blocks each that share the quartet's primitives, from block start[k] on; the
-    // largest quartets have the highest k
+    // segments of the launch (tile_segments), 2^k blocks that share a quartet's primitives
+    // in segment k; block0: a launch's first block, where they do not fit one grid
     int nseg = 1;
-    long long start[TILE_SEGS + 1] = {};
-    int first[TILE_SEGS + 1] = {};
+    long long block0 = 0;
+    long long start[SEG_POW] = {};
+    long long first[SEG_POW] = {};
     const double* D = nullptr;
     double cj = 0.0, ck = 0.0;
     double* grad = nullptr;  // 3N, atomic adds
@@ -760,12 +760,14 @@ __global__ void __launch_bounds__(C::NT, TileBounds<C>::MINB) k_tile(TileArgs ta
     const typename Ket::Tab& tk = g_tile_tab<C::lc, C::ld>;
     const EriArgs& a = ta.e;
     int seg = ta.nseg - 1;  // block-uniform
-    while (seg > 0 && (long long)blockIdx.x >= ta.start[seg - 1]) --seg;
-    const int rel = (int)(blockIdx.x - ta.start[seg]), parts = 1 << seg;
+    const long long bid = ta.block0 + blockIdx.x;
+    while (seg > 0 && bid >= ta.start[seg - 1]) --seg;
+    const long long rel = bid - ta.start[seg];
+    const int parts = 1 << seg;
     const long long n = a.n, qi = list_index(a, ta.first[seg] + (rel >> seg));
     const int2 pq = a.quartets[qi];
     const int ntot = a.pairs[pq.x].nprim * a.pairs[pq.y].nprim;
-    const int part = rel & (parts - 1), stride = parts * C::PB;
+    const int part = (int)rel & (parts - 1), stride = parts * C::PB;
     if (part * C::PB >= ntot) return;  // whole block
     if (tid < 24) {
         reinterpret_cast<int*>(&w.P)[tid] = reinterpret_cast<const int*>(a.pairs + pq.x)[tid];
@@ -913,41 +915,27 @@ __global__ void __launch_bounds__(C::NT, TileBounds<C>::MINB) k_tile(TileArgs ta
     }
 }
 
-// Blocks of a class.  A quartet has 1 to 4,096 primitives; with one block each the largest
-// ones were the tail of every launch (ten atoms, (22|21): the FP64 pipe 45% busy while
-// blocks ran, 26% over the launch).  A block takes at most `share` primitives: an eighth
-// of what each of the GPU's block slots gets in all, and two batches at least (gradient:
-// 48 primitives, about what its transfers of Gamma cost).  prefix[k]
-// counts the quartets with more than 2^k primitives in the processing order, which has
-// the largest first; without one (null: equal counts, or a list of its own) all quartets
-// are taken as the largest.
+// Blocks of a class.  With one block per quartet the largest ones were the tail of every
+// launch (ten atoms, (22|21): the FP64 pipe 45% busy while blocks ran, 26% over the
+// launch).  A block takes at most `share` primitives: an eighth of what each of the GPU's
+// block slots gets in all, and two batches at least (gradient: 48 primitives, about what
+// its transfers of Gamma cost).  prefix[k] counts the quartets with more than 2^k
+// primitives in the processing order (null: no order).
 template <class C>
-void launch_tile(TileArgs& ta, int mode, long long nq, long long prims, int max_prims, const int* prefix, cudaStream_t s) {
+void launch_tile(TileArgs& ta, int mode, long long nq, long long prims, long long max_prims, const long long* prefix,
+                 cudaStream_t s) {
     if (nq <= 0) return;
     auto k = k_tile<C>;
     if (C::SMEM > 40 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
     const long long share = std::max<long long>(C::DER ? std::max(2 * C::PB, 48) : 2 * C::PB,
                                                 prims / (148LL * TileBounds<C>::MINB * 8) + 1);
-    int low = 0;  // share rounded down to a power of two
-    while (low < TILE_SEGS - 1 && (2LL << low) <= share) ++low;
-    ta.nseg = 1;
-    if (mode != MODE_SCHWARZ)
-        while (ta.nseg < TILE_SEGS && (max_prims - 1) >> (low + ta.nseg - 1)) ++ta.nseg;
-    // segment j: more than 2^(low + j - 1) primitives (none has more than the last's)
-    long long blocks = 0;
-    int from = 0;
-    for (int j = ta.nseg - 1; j >= 0; --j) {
-        ta.first[j] = from;
-        ta.start[j] = blocks;
-        int to = (int)nq;
-        if (j > 0 && prefix) to = low + j - 1 < TILE_SEGS ? prefix[low + j - 1] : 0;
-        to = std::max(from, to);
-        blocks += (long long)(to - from) << j;
-        from = to;
-    }
+    long long blocks;
+    ta.nseg = tile_segments(nq, share, max_prims, prefix, mode == MODE_SCHWARZ ? 1 : 1 << 24, ta.first, ta.start, &blocks);
     if (ta.nseg > 1 && !C::DER && mode == MODE_UNIQUE)
         cudaMemsetAsync(ta.e.out + ta.e.base, 0, sizeof(double) * nq * C::NCOMP, s);
-    k<<<dim3((unsigned)blocks, 1, C::NPASS), C::NT, C::SMEM, s>>>(ta, mode);
+    constexpr long long GRID = 1LL << 30;
+    for (ta.block0 = 0; ta.block0 < blocks; ta.block0 += GRID)
+        k<<<dim3((unsigned)std::min(GRID, blocks - ta.block0), 1, C::NPASS), C::NT, C::SMEM, s>>>(ta, mode);
 }
 #endif  // TILE_HOST
 
