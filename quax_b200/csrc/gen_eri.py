@@ -1163,19 +1163,20 @@ def gen_sl(here, qc):
 
 
 def gen_tile(here):
-    """One translation unit per class up to RYS_LMAX with the tile engine's launcher
-    qx_launch_tile_<id>(args, kind, mode, nquartets, primitive quartets, the largest
-    quartet's, counts above powers of two, stream)."""
+    """One translation unit per class up to RYS_LMAX with the launcher of its plain
+    (qx_plain.cuh) and adjoint-gradient (qx_tile.cuh) kernels, qx_launch_tile_<id>(args,
+    kind, mode, nquartets, primitive quartets, the largest quartet's, counts above powers
+    of two, stream)."""
     qc = quartet_classes(RYS_LMAX)
     for i, (a, b, c, d) in enumerate(qc):
         L = ["// Generated by quax_b200/csrc/gen_eri.py -- do not edit by hand.",
              f"// Tile-engine launchers of class ({a}{b}|{c}{d}).",
-             '#include "../qx_tile.cuh"',
+             '#include "../qx_plain.cuh"',
              f"void qx_launch_tile_{i:02d}(qx::TileArgs& ta, int kind, int mode, long long nq, long long prims, "
-             "long long max_prims, const long long* prefix, cudaStream_t s) {"]
-        for k in ("TK_PLAIN", "TK_GRAD"):
-            L.append(f"    if (kind == qx::{k}) return qx::launch_tile<qx::TileCls<{a}, {b}, {c}, {d}, qx::{k}>>"
-                     "(ta, mode, nq, prims, max_prims, prefix, s);")
+             "long long max_prims, const long long* prefix, cudaStream_t s) {",
+             f"    if (kind == qx::TK_PLAIN) qx::launch_plain<qx::PlainCls<{a}, {b}, {c}, {d}>>"
+             "(ta, mode, nq, prims, max_prims, prefix, s);",
+             f"    else qx::launch_tile<qx::TileCls<{a}, {b}, {c}, {d}, qx::TK_GRAD>>(ta, nq, prims, max_prims, prefix, s);"]
         L += ["}"]
         with _Out(os.path.join(here, "gen", f"k_tile_{i:02d}.cu")) as f:
             f.write("\n".join(L) + "\n")

@@ -153,8 +153,8 @@ QX_FOR_EACH_DSPLIT(QX_DECL_DS)
 // cooperative HRR; ENG_WSPLIT (plain): the same VRR split + the warp HRR.
 // ENG_DSPLIT (derivatives): the split VRR into item-order accumulators + the warp
 // kernel's own HRR and epilogue.
-// ENG_RYS: Rys quadrature -- the tile kernels (qx_tile.cuh) for plain integrals and the
-// adjoint gradient, qx_rys.cuh for derivative tensors and tiles; the only engine of the
+// ENG_RYS: Rys quadrature -- qx_plain.cuh for plain integrals, qx_tile.cuh for the adjoint
+// gradient, qx_rys.cuh for derivative tensors and tiles; the only engine of the
 // classes with an f shell.
 enum { ENG_SL = 0, ENG_WARP = 1, ENG_COOP = 2, ENG_WVRR = 3, ENG_WSPLIT = 4, ENG_DSPLIT = 5, ENG_RYS = 6 };
 int qx_der_index(int cls);
@@ -797,6 +797,12 @@ extern "C" int qx_initialize(int natom, const double* coords, int nshell, const 
             const int cls = quartet_class(pc, pc);
             const int keep_wpq = h->wpq[cls];
             h->wpq[cls] = 4;
+            ClassWork& w = h->work[cls];  // this launch's primitives; the class's own follow
+            for (const int2& q : diag[pc]) {
+                const long long k = (long long)h->pairs[q.x].nprim * h->pairs[q.x].nprim;
+                w.prims += k;
+                w.max_prims = std::max(w.max_prims, k);
+            }
             int rc = run_class(h, cls, MODE_SCHWARZ, d_dq + o, (long long)diag[pc].size(), d_kp, 0, 0, 0,
                                g_class_scratch[cls] ? 0 : 5);
             h->wpq[cls] = keep_wpq;
@@ -1645,20 +1651,26 @@ extern "C" int qx_oei_deriv_core(qx_handle* h, int order, double* dS, double* dT
 }
 
 // ---------------------------------------------------------------- class info ---
-// Algorithmic FP64 FLOPs of one primitive quartet of the tile programs (plain:
-// deriv = 0; adjoint gradient: deriv = 1), counted per step of qx_tile.cuh: the 2n
-// Chebyshev series (13 Clenshaw steps, 4 flops each), the 3n two-dimensional tables (5
-// flops per entry), and per f and root 2 flops per (e0|f0) value and 1 per (ex, ey) pair;
-// the gradient 6 per value, 5 per pair, and 2 for each of the lowered terms of the three
-// directions (bra and ket) and of E0.
+// Algorithmic FP64 FLOPs of one primitive quartet of the Rys programs, counted per step:
+// the 2n Chebyshev series (13 Clenshaw steps, 4 flops each) and the 3n two-dimensional
+// tables (5 flops per entry); plain (deriv = 0, qx_plain.cuh) 2 flops per transferred
+// entry and 3 per component and root; adjoint gradient (deriv = 1, qx_tile.cuh) per f and
+// root 6 flops per (e0|f0) value, 5 per (ex, ey) pair, and 2 for each of the lowered terms
+// of the three directions (bra and ket) and of E0.
 static double rys_prim_flops(const int* l, int deriv) {
     const int L = l[0] + l[1] + l[2] + l[3], NR = (L + deriv) / 2 + 1;
     const int HI = l[0] + l[1], NI = HI + 1, NK = l[2] + l[3] + 1;
+    double f = 2.0 * NR * 52.0 + 3.0 * NR * NI * NK * 5.0;
+    if (!deriv) {
+        double ncomp = 1.0;
+        for (int i = 0; i < 4; ++i) ncomp *= (l[i] + 1) * (l[i] + 2) / 2;
+        for (int b = 1; b <= l[1]; ++b) f += 3.0 * NR * (NI - b) * NK * 2.0;
+        for (int d = 1; d <= l[3]; ++d) f += 3.0 * NR * (l[0] + 1) * (l[1] + 1) * (NK - d) * 2.0;
+        return f + ncomp * NR * 3.0;
+    }
     auto hoff = [](int x) { return x * (x + 1) * (x + 2) / 6; };
     const double NE = hoff(HI + 1) - hoff(l[0]), NF = hoff(l[2] + l[3] + 1) - hoff(l[2]);
     const double pairs = (HI + 1) * (HI + 2) / 2;
-    const double f = 2.0 * NR * 52.0 + 3.0 * NR * NI * NK * 5.0;
-    if (!deriv) return f + NF * NR * (2.0 * NE + pairs);
     return f + NF * NR * (6.0 * NE + 5.0 * pairs + 14.0 * (HI + 1));
 }
 

@@ -53,8 +53,8 @@ constexpr int RYS_TABLE_DOUBLES = QX_RYS_TAB_SIZE + 2 * QX_RYS_ASYM_SIZE;
 // derivative order the quadrature must integrate, and the per-direction 1-D
 // derivative tables the products read.
 // The device kernel runs the Hessian-vector product, the gradient tile and the derivative
-// tensors; plain integrals and the adjoint gradient run in qx_tile.cuh, and their product
-// steps here serve the host check of the tables.
+// tensors; plain integrals run in qx_plain.cuh and the adjoint gradient in qx_tile.cuh, and
+// their product steps here serve the host checks of the tables and of qx_plain.cuh.
 enum { RK_PLAIN = 0, RK_GRAD = 1, RK_HVP = 2, RK_GRADT = 3, RK_DER1 = 11, RK_DER2 = 12, RK_DER3 = 13, RK_DER4 = 14 };
 QX_HD constexpr bool rys_is_grad(int kind) { return kind == RK_GRAD; }
 
@@ -840,7 +840,7 @@ __device__ __forceinline__ void rys_primitive(const RysArgs& ra, const PrimPair&
 template <int LA, int LB, int LC, int LD, int KIND>
 __global__ void __launch_bounds__(RysCls<LA, LB, LC, LD, KIND>::BS, RysCls<LA, LB, LC, LD, KIND>::MINB)
     k_rys(RysArgs ra, long long nwork) {
-    static_assert(KIND == RK_HVP || KIND == RK_GRADT || KIND >= RK_DER1, "plain integrals and the gradient: qx_tile.cuh");
+    static_assert(KIND == RK_HVP || KIND == RK_GRADT || KIND >= RK_DER1, "plain integrals: qx_plain.cuh, the gradient: qx_tile.cuh");
     using C = RysCls<LA, LB, LC, LD, KIND>;
     constexpr int TS = C::TS, TPB = C::TPB, NCPT = C::NCPT;
     extern __shared__ double rys_sm[];

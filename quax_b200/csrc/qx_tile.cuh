@@ -1,43 +1,46 @@
-// qx_tile.cuh -- Rys quadrature with the transfer after the contraction: plain
-// integrals and the adjoint gradient, every class up to (ff|ff).
+// qx_tile.cuh -- the adjoint gradient by Rys quadrature with the transfer after the
+// contraction, every class up to (ff|ff); and the pieces it shares with the plain
+// integrals (qx_plain.cuh).
 //
 // Method.  A primitive [e0|f0] with all quanta on the first centre of each side is
 // sum_r w_r Ix(ex,fx) Iy(ey,fy) Iz(ez,fz) over the Rys nodes (Dupuis, Rys & King, J. Chem.
 // Phys. 65, 111 (1976)); the 1-D factors follow the two-term recurrences of qx_rys.cuh.
 // The transfer (ab| = sum_k C(b,k) AB^{b-k} (a+k,0| (Head-Gordon & Pople, J. Chem. Phys.
-// 89, 5777 (1988), in closed form) does not depend on the primitives, so it is applied
-// once per contracted quartet, and the primitive loop only ever sees the (e0|f0) values
-// U[e,f]: 1,426 for (32|22) where the (ab|cd) block has 2,160, and two operations per
-// value and root.
+// 89, 5777 (1988), in closed form) does not depend on the primitives.
 //
-// The adjoint gradient never forms derivative integrals.  With G[e,f] = the transfer's
-// transpose applied to Gamma, E = sum G[e,f] U[e,f].  Per primitive and root a thread sums
-// G over two directions, gx[ex] = sum G Iy Iz, and one direction's short sums give E0 =
-// sum G V, LA = sum G e V(e-1) and LC = sum G f V(f-1).  Moving the bra as a whole changes
-// only P - Q; differentiating the recurrences,
+// The gradient never forms derivative integrals.  With G[e,f] = the transfer's transpose
+// applied to Gamma, and U[e,f] the (e0|f0) values, E = sum G[e,f] U[e,f].  Per primitive
+// and root a thread sums G over two directions, gx[ex] = sum G Iy Iz, and one direction's
+// short sums give E0 = sum G V, LA = sum G e V(e-1) and LC = sum G f V(f-1).  Moving the
+// bra as a whole changes only P - Q; differentiating the recurrences,
 //   t = sum_r (-2 rho u PQ E0 - u q/(p+q) LA + u p/(p+q) LC)_r  (p, q: the two zetas),
 // and the derivatives of the Gaussians at fixed P - Q are polynomials again:
 //   dE/dA = sum_prim (a/p) t - (b/p) (LA + 2 a AB E0) + X_AB,   dE/dB = t - dE/dA
 //   dE/dC = sum_prim -(c/q) t - (d/q) (LC + 2 c CD E0) + X_CD,  dE/dD = -t - dE/dC
 // with X_AB = sum (dG/dAB) U.  No term is raised, so no tight exponent multiplies a
-// difference of moments, as 2 b (V(e+1) + AB V(e)) would for a tight b.
+// difference of moments, as 2 b (V(e+1) + AB V(e)) would for a tight b: on eight random
+// molecules with s to f shells the gradient lies 1e-15 to 9e-14 of its largest entry from
+// an 80-bit evaluation, the programs it replaces 4e-15 to 2e-11.  (The transfer after the
+// contraction does cost the (33|xx) classes digits, up to 1e-12 of the class's own
+// contribution, where the others lost more.)
 //
 // Organisation.  A block owns (quartet, part of its primitives).  Per batch of PB
 // primitives: the nodes and weights (one thread per function), the 2-D tables in shared
 // memory (one thread per primitive, root and direction), then the sums: a lane owns one
 // f and one of NP primitives of the batch, a warp one chunk of the e's -- a set of ex
 // values, compile time, so that a chunk's values live in registers and one load of a
-// column serves them all.  Parts of a quartet add into the outputs with atomics: every
-// output is linear in the primitives.
+// column serves them all.  Parts of a quartet add into the gradient with atomics.
+//
+// TK_PLAIN: the same transfer forwards, in host code only; its phases serve the host check
+// of the tables (the plain kernels transfer each 1-D factor instead, for accuracy).
 //
 // What bounds it: the FP64 pipe in the sums (about 2/3 of the instructions of the large
-// classes); the kernels it replaces kept the (a,b,c,d) tables of every root and read three
-// (gradient: 21) of their entries per component and root, which bound them on shared
-// memory, and walked all primitives of a quartet on one team.
+// classes); the kernels it replaces kept the (a,b,c,d) tables of every root and read 21 of
+// their entries per component and root, which bound them on shared memory, and walked all
+// primitives of a quartet on one team.
 #pragma once
 #include <algorithm>
 
-#include "qx_jk.cuh"
 #include "qx_rys.cuh"
 #include "qx_segments.h"
 
@@ -126,6 +129,38 @@ enum { TK_PLAIN = 0, TK_GRAD = 1 };
 // ------------------------------------------------------------------ one class --
 constexpr int TILE_SMEM_TARGET = 72 * 1024;  // tables of a batch (bytes)
 constexpr int TILE_MAXW = 8;                 // warps per block
+constexpr long long TILE_GRID = 1LL << 30;   // blocks per launch
+
+// Warps per chunk: the fewest that hold all nf lanes, more while their lanes fill better
+// and while no more than 16 primitives are summed side by side (a quartet has a few dozen).
+QX_HD constexpr int tl_wpc(int nf, int wmin, int nchb) {
+    int best = wmin;
+    double bu = 0.0;
+    for (int w = wmin; w * nchb <= TILE_MAXW; ++w) {
+        if (w > wmin && 32 * w / nf > 16) break;
+        const double u = (double)(32 * w / nf * nf) / (32 * w) + (w * nchb <= 4 ? 0.04 * w * nchb : 0.0);
+        if (u > bu + 0.08) {
+            bu = u;
+            best = w;
+        }
+    }
+    return best;
+}
+// Primitives per batch: a multiple of np whose units fill the block's threads best.
+QX_HD constexpr int tl_pb(int np, int nr, int nt, int per_prim) {
+    const int cap = TILE_SMEM_TARGET / 8 / per_prim;
+    int best = np;
+    double bu = 0.0;
+    for (int p = np; p <= cap && p <= 128; p += np) {
+        const int u = 3 * nr * p, rounds = (u + nt - 1) / nt;
+        const double f = (double)u / (rounds * nt) - 0.02 * rounds;
+        if (f > bu + 0.02) {
+            bu = f;
+            best = p;
+        }
+    }
+    return best;
+}
 
 template <int LA, int LB, int LC, int LD, int KIND>
 struct TileCls {
@@ -181,41 +216,11 @@ struct TileCls {
     }
     QX_HD static constexpr int MASK(int k) { return chunks().mask[k]; }
     static constexpr int NSLOT = chunks().most;
-    // warps per chunk: the fewest that hold all f, more while their lanes fill better and
-    // while no more than 16 primitives are summed side by side (a quartet has a few dozen)
-    QX_HD static constexpr int wpc() {
-        int best = WMIN;
-        double bu = 0.0;
-        for (int w = WMIN; w * NCHB <= TILE_MAXW; ++w) {
-            if (w > WMIN && 32 * w / NF > 16) break;
-            const double u = (double)(32 * w / NF * NF) / (32 * w) + (w * NCHB <= 4 ? 0.04 * w * NCHB : 0.0);
-            if (u > bu + 0.08) {
-                bu = u;
-                best = w;
-            }
-        }
-        return best;
-    }
-    static constexpr int WPC = wpc();
+    static constexpr int WPC = tl_wpc(NF, WMIN, NCHB);
     static constexpr int W = WPC * NCHB, NT = 32 * W;
     static constexpr int NP = 32 * WPC / NF;  // primitives of a batch summed side by side
     static constexpr int PER_PRIM = 3 * NR * UNIT;  // table entries of one primitive
-    // primitives per batch: a multiple of NP whose units fill the block's threads best
-    QX_HD static constexpr int pb() {
-        const int cap = TILE_SMEM_TARGET / 8 / PER_PRIM;
-        int best = NP;
-        double bu = 0.0;
-        for (int p = NP; p <= cap && p <= 128; p += NP) {
-            const int u = 3 * NR * p, rounds = (u + NT - 1) / NT;
-            const double f = (double)u / (rounds * NT) - 0.02 * rounds;
-            if (f > bu + 0.02) {
-                bu = f;
-                best = p;
-            }
-        }
-        return best;
-    }
-    static constexpr int PB = pb();
+    static constexpr int PB = tl_pb(NP, NR, NT, PER_PRIM);
     // shared memory, in doubles: the persistent part, then a region that holds the
     // batch's tables, or (before and after the primitives) the transfer's arrays
     static constexpr int CO = (Bra::NCOMBO + Ket::NCOMBO) * (DER ? 4 : 1);
@@ -244,9 +249,9 @@ struct TileCls {
 struct TileArgs {
     EriArgs e;
     const double* rys = nullptr;
-    // segments of the launch (tile_segments), 2^k blocks that share a quartet's primitives
-    // in segment k; block0: a launch's first block, where they do not fit one grid
-    int nseg = 1;
+    // segments of the launch (tile_segments), 2^(lg0 + k) blocks that share a quartet's
+    // primitives in segment k; block0: a launch's first block, where they do not fit one grid
+    int nseg = 1, lg0 = 0;
     long long block0 = 0;
     long long start[SEG_POW] = {};
     long long first[SEG_POW] = {};
@@ -412,7 +417,7 @@ QX_HD inline void tl_x_ket(const typename C::Ket::Tab& t, const double* co, cons
     }
 }
 
-// Forward transfer of the plain kind: H[ab][f] from U, and one component from H.
+// Forward transfer (TK_PLAIN): H[ab][f] from U, and one component from H.
 template <class C>
 QX_HD inline void tl_fwd_bra(const typename C::Bra::Tab& t, const double* co, const double* U, double* H, int tid,
                              int nth) {
@@ -738,8 +743,33 @@ struct TileBounds {
     static constexpr int MINB = B0 < 1 ? 1 : (B0 > 16 ? 16 : B0);
 };
 
+struct TileBlock {
+    long long quartet;  // position in the processing order
+    int part, parts;
+};
+__device__ __forceinline__ TileBlock tile_block(const TileArgs& ta) {
+    int seg = ta.nseg - 1;  // block-uniform
+    const long long bid = ta.block0 + blockIdx.x;
+    while (seg > 0 && bid >= ta.start[seg - 1]) --seg;
+    const long long rel = bid - ta.start[seg];
+    const int lg = ta.lg0 + seg;
+    return {ta.first[seg] + (rel >> lg), (int)(rel & ((1LL << lg) - 1)), 1 << lg};
+}
+
+// The quartet's pair records to shared memory.
+template <int NT>
+__device__ __forceinline__ void tile_pairs(const EriArgs& a, int2 pq, TileQuartet& w, int tid) {
+    if (tid < 24) {
+        reinterpret_cast<int*>(&w.P)[tid] = reinterpret_cast<const int*>(a.pairs + pq.x)[tid];
+    } else if (tid < 48 && NT >= 48) {
+        reinterpret_cast<int*>(&w.Q)[tid - 24] = reinterpret_cast<const int*>(a.pairs + pq.y)[tid - 24];
+    }
+    if (NT < 48 && tid < 24) reinterpret_cast<int*>(&w.Q)[tid] = reinterpret_cast<const int*>(a.pairs + pq.y)[tid];
+}
+
 template <class C>
-__global__ void __launch_bounds__(C::NT, TileBounds<C>::MINB) k_tile(TileArgs ta, int mode) {
+__global__ void __launch_bounds__(C::NT, TileBounds<C>::MINB) k_tile(TileArgs ta) {
+    static_assert(C::DER, "plain integrals: qx_plain.cuh");
     using Bra = typename C::Bra;
     using Ket = typename C::Ket;
     constexpr int NT = C::NT;
@@ -759,33 +789,20 @@ __global__ void __launch_bounds__(C::NT, TileBounds<C>::MINB) k_tile(TileArgs ta
     const typename Bra::Tab& tb = g_tile_tab<C::la, C::lb>;
     const typename Ket::Tab& tk = g_tile_tab<C::lc, C::ld>;
     const EriArgs& a = ta.e;
-    int seg = ta.nseg - 1;  // block-uniform
-    const long long bid = ta.block0 + blockIdx.x;
-    while (seg > 0 && bid >= ta.start[seg - 1]) --seg;
-    const long long rel = bid - ta.start[seg];
-    const int parts = 1 << seg;
-    const long long n = a.n, qi = list_index(a, ta.first[seg] + (rel >> seg));
-    const int2 pq = a.quartets[qi];
+    const TileBlock at = tile_block(ta);
+    const long long n = a.n;
+    const int2 pq = a.quartets[list_index(a, at.quartet)];
     const int ntot = a.pairs[pq.x].nprim * a.pairs[pq.y].nprim;
-    const int part = (int)rel & (parts - 1), stride = parts * C::PB;
+    const int part = at.part, stride = at.parts * C::PB;
     if (part * C::PB >= ntot) return;  // whole block
-    if (tid < 24) {
-        reinterpret_cast<int*>(&w.P)[tid] = reinterpret_cast<const int*>(a.pairs + pq.x)[tid];
-    } else if (tid < 48 && NT >= 48) {
-        reinterpret_cast<int*>(&w.Q)[tid - 24] = reinterpret_cast<const int*>(a.pairs + pq.y)[tid - 24];
-    }
-    if (NT < 48 && tid < 24) reinterpret_cast<int*>(&w.Q)[tid] = reinterpret_cast<const int*>(a.pairs + pq.y)[tid];
+    tile_pairs<NT>(a, pq, w, tid);
     __syncthreads();
     const bool sPQ = pq.x != pq.y;
-    if constexpr (C::DER) {
-        if (w.P.atom1 == w.P.atom2 && w.P.atom1 == w.Q.atom1 && w.P.atom1 == w.Q.atom2) return;
-    } else {
-        if (mode == MODE_JK && jk_screened(a, pq, w.P, w.Q)) return;  // block-uniform
-    }
+    if (w.P.atom1 == w.P.atom2 && w.P.atom1 == w.Q.atom1 && w.P.atom1 == w.Q.atom2) return;
     {
         const double AB[3] = {w.P.ABx, w.P.ABy, w.P.ABz}, CD[3] = {w.Q.ABx, w.Q.ABy, w.Q.ABz};
-        tl_coefs<Bra, C::DER>(tb, AB, coA, tid, NT);
-        tl_coefs<Ket, C::DER>(tk, CD, coC, tid, NT);
+        tl_coefs<Bra, true>(tb, AB, coA, tid, NT);
+        tl_coefs<Ket, true>(tk, CD, coC, tid, NT);
     }
     const TileRole<C> role(tid, C::NPASS > 1 ? blockIdx.z : 0);
     TileThread<C> th;
@@ -794,16 +811,14 @@ __global__ void __launch_bounds__(C::NT, TileBounds<C>::MINB) k_tile(TileArgs ta
 #pragma unroll
     for (int i = 0; i < 9; ++i) th.g[i] = 0.0;
     TileGamma<C> gam = tl_gamma<C>(den, w.P, w.Q, sPQ, ta.cj, ta.ck);
-    if constexpr (C::DER) {
-        tl_density<C>(ta.D, n, w.P, w.Q, den, tid, NT);
-        __syncthreads();
-        tl_gam_ket<C>(tk, coC, gam, Hx, tid, NT);
-        __syncthreads();
-        tl_gam_bra<C>(tb, coA, Hx, Uy, tid, NT);
-        __syncthreads();
-        tl_load<C, 0>(role.on ? role.chunk : 0, Uy, role.f, th);
-        __syncthreads();
-    }
+    tl_density<C>(ta.D, n, w.P, w.Q, den, tid, NT);
+    __syncthreads();
+    tl_gam_ket<C>(tk, coC, gam, Hx, tid, NT);
+    __syncthreads();
+    tl_gam_bra<C>(tb, coA, Hx, Uy, tid, NT);
+    __syncthreads();
+    tl_load<C, 0>(role.on ? role.chunk : 0, Uy, role.f, th);
+    __syncthreads();
     const PrimPair* bra = a.prims + w.P.prim_off;
     const PrimPair* ket = a.prims + w.Q.prim_off;
     const int fx = tk.ex[role.f], fy = tk.ey[role.f], fz = tk.ez[role.f];
@@ -818,10 +833,9 @@ __global__ void __launch_bounds__(C::NT, TileBounds<C>::MINB) k_tile(TileArgs ta
             for (int p = role.sub; p < nb; p += C::NP)
                 tl_prim_chunk<C, 0>(role.chunk, tab + (size_t)p * C::PER_PRIM, uwp + 2 * C::NR * p, fx, fy, fz,
                                     scp + C::SCP * p, w, th);
-        if (C::DER) {  // the next batch's nodes and scalars beside these
-            scp = scp == sc ? sc + C::NSC / 2 : sc;
-            uwp = uwp == uw ? uw + C::UWB : uw;
-        }
+        // the next batch's nodes and scalars beside these
+        scp = scp == sc ? sc + C::NSC / 2 : sc;
+        uwp = uwp == uw ? uw + C::UWB : uw;
     }
     __syncthreads();
     // U of the NP primitives side by side -> Uy
@@ -848,94 +862,50 @@ __global__ void __launch_bounds__(C::NT, TileBounds<C>::MINB) k_tile(TileArgs ta
     } else {
         __syncthreads();
     }
-    if constexpr (C::DER) {
-        if constexpr (C::lb > 0) {
-            tl_gam_ket<C>(tk, coC, gam, Hx, tid, NT);
-            __syncthreads();
-            tl_x_bra<C>(tb, coA, Uy, Hx, th.g, tid, NT);
-            if (C::ld > 0) __syncthreads();
-        }
-        if constexpr (C::ld > 0) {
-            tl_gam_bra2<C>(tb, coA, gam, Hx, tid, NT);
-            __syncthreads();
-            tl_x_ket<C>(tk, coC, Uy, Hx, th.g, tid, NT);
-        }
+    if constexpr (C::lb > 0) {
+        tl_gam_ket<C>(tk, coC, gam, Hx, tid, NT);
+        __syncthreads();
+        tl_x_bra<C>(tb, coA, Uy, Hx, th.g, tid, NT);
+        if (C::ld > 0) __syncthreads();
+    }
+    if constexpr (C::ld > 0) {
+        tl_gam_bra2<C>(tb, coA, gam, Hx, tid, NT);
+        __syncthreads();
+        tl_x_ket<C>(tk, coC, Uy, Hx, th.g, tid, NT);
+    }
 #pragma unroll
-        for (int i = 0; i < 9; ++i) {
-            for (int off = 16; off > 0; off >>= 1) th.g[i] += __shfl_xor_sync(0xffffffffu, th.g[i], off);
-            if ((tid & 31) == 0) red[(tid >> 5) * 9 + i] = th.g[i];
-        }
-        __syncthreads();
-        if (tid < 12) {
-            const int x = tid % 3, c = tid / 3;
-            double v = 0.0;
-            for (int k = 0; k < C::W; ++k)
-                v += c < 3 ? red[k * 9 + tid] : -(red[k * 9 + x] + red[k * 9 + 3 + x] + red[k * 9 + 6 + x]);
-            const int at = c == 0 ? w.P.atom1 : (c == 1 ? w.P.atom2 : (c == 2 ? w.Q.atom1 : w.Q.atom2));
-            atomicAdd(ta.grad + 3 * at + x, v);
-        }
-    } else {
-        constexpr int NA = Bra::N1, NB = Bra::N2, NC = Ket::N1, ND = Ket::N2;
-        tl_fwd_bra<C>(tb, coA, Uy, Hx, tid, NT);
-        __syncthreads();
-        const bool s12 = w.P.s1 != w.P.s2, s34 = w.Q.s1 != w.Q.s2;
-        if (mode == MODE_SCHWARZ) {
-            double mx = 0.0;
-            if constexpr (NA * NB == NC * ND)
-                for (int o = tid; o < NA * NB; o += NT) mx = fmax(mx, fabs(tl_fwd_ket<C>(tk, coC, Hx, o, o)));
-            for (int off = 16; off > 0; off >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-            if ((tid & 31) == 0) red[tid >> 5] = mx;
-            __syncthreads();
-            if (tid == 0) {
-                for (int k = 1; k < C::W; ++k) mx = fmax(mx, red[k]);
-                a.out[pq.x] = mx;
-            }
-        } else if (mode == MODE_JK) {
-            double* out = region;
-            for (int o = tid; o < C::NCOMP; o += NT) out[o] = tl_fwd_ket<C>(tk, coC, Hx, o / (NC * ND), o % (NC * ND));
-            __syncthreads();
-            jk_block<NA, NB, NC, ND>(a.out, a.out2, a.dens, n, w.P, w.Q, s12, s34, sPQ, tid, NT,
-                                     [&](int o) { return out[o]; });
-        } else {
-            const bool add = parts > 1;  // parts of a quartet meet in zeroed outputs
-            for (int o = tid; o < C::NCOMP; o += NT) {
-                const int ab = o / (NC * ND), cd = o - ab * (NC * ND);
-                const double v = tl_fwd_ket<C>(tk, coC, Hx, ab, cd);
-                if (mode == MODE_UNIQUE) {
-                    double* u = a.out + a.base + (long long)o * a.nq + qi;
-                    if (add) atomicAdd(u, v);
-                    else *u = v;
-                    continue;
-                }
-                const long long i = w.P.bf1 + ab / NB, j = w.P.bf2 + ab % NB, k = w.Q.bf1 + cd / ND, l = w.Q.bf2 + cd % ND;
-                if (add) atomic_images_w(a.out, n, i, j, k, l, s12, s34, sPQ, v);
-                else dense_images(a.out, n, i, j, k, l, s12, s34, sPQ, v);
-            }
-        }
+    for (int i = 0; i < 9; ++i) {
+        for (int off = 16; off > 0; off >>= 1) th.g[i] += __shfl_xor_sync(0xffffffffu, th.g[i], off);
+        if ((tid & 31) == 0) red[(tid >> 5) * 9 + i] = th.g[i];
+    }
+    __syncthreads();
+    if (tid < 12) {
+        const int x = tid % 3, c = tid / 3;
+        double v = 0.0;
+        for (int k = 0; k < C::W; ++k)
+            v += c < 3 ? red[k * 9 + tid] : -(red[k * 9 + x] + red[k * 9 + 3 + x] + red[k * 9 + 6 + x]);
+        const int atom = c == 0 ? w.P.atom1 : (c == 1 ? w.P.atom2 : (c == 2 ? w.Q.atom1 : w.Q.atom2));
+        atomicAdd(ta.grad + 3 * atom + x, v);
     }
 }
 
 // Blocks of a class.  With one block per quartet the largest ones were the tail of every
 // launch (ten atoms, (22|21): the FP64 pipe 45% busy while blocks ran, 26% over the
 // launch).  A block takes at most `share` primitives: an eighth of what each of the GPU's
-// block slots gets in all, and two batches at least (gradient: 48 primitives, about what
-// its transfers of Gamma cost).  prefix[k] counts the quartets with more than 2^k
+// block slots gets in all, and two batches and 48 primitives at least (about what the
+// transfers of Gamma cost).  prefix[k] counts the quartets with more than 2^k
 // primitives in the processing order (null: no order).
 template <class C>
-void launch_tile(TileArgs& ta, int mode, long long nq, long long prims, long long max_prims, const long long* prefix,
+void launch_tile(TileArgs& ta, long long nq, long long prims, long long max_prims, const long long* prefix,
                  cudaStream_t s) {
     if (nq <= 0) return;
     auto k = k_tile<C>;
     if (C::SMEM > 40 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
-    const long long share = std::max<long long>(C::DER ? std::max(2 * C::PB, 48) : 2 * C::PB,
-                                                prims / (148LL * TileBounds<C>::MINB * 8) + 1);
+    const long long share = std::max<long long>(std::max(2 * C::PB, 48), prims / (148LL * TileBounds<C>::MINB * 8) + 1);
     long long blocks;
-    ta.nseg = tile_segments(nq, share, max_prims, prefix, mode == MODE_SCHWARZ ? 1 : 1 << 24, ta.first, ta.start, &blocks);
-    if (ta.nseg > 1 && !C::DER && mode == MODE_UNIQUE)
-        cudaMemsetAsync(ta.e.out + ta.e.base, 0, sizeof(double) * nq * C::NCOMP, s);
-    constexpr long long GRID = 1LL << 30;
-    for (ta.block0 = 0; ta.block0 < blocks; ta.block0 += GRID)
-        k<<<dim3((unsigned)std::min(GRID, blocks - ta.block0), 1, C::NPASS), C::NT, C::SMEM, s>>>(ta, mode);
+    ta.nseg = tile_segments(nq, share, max_prims, prefix, 1 << 24, ta.first, ta.start, &blocks);
+    for (ta.block0 = 0; ta.block0 < blocks; ta.block0 += TILE_GRID)
+        k<<<dim3((unsigned)std::min(TILE_GRID, blocks - ta.block0), 1, C::NPASS), C::NT, C::SMEM, s>>>(ta);
 }
 #endif  // TILE_HOST
 
