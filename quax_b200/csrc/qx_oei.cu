@@ -22,6 +22,7 @@
 //             derivative of the nuclear term with respect to the nucleus C follows
 //             from translational invariance of each term: d/dC = -(d/dA + d/dB).
 // Every block is written for both (i,j) and (j,i) by the lane that owns it.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -291,7 +292,11 @@ __global__ void __launch_bounds__(128) k_oei(OeiArgs a) {
 // (primitive pair, root) units NAI_UB at a time: three lanes per unit build the three
 // directions' 1-D tables (values, and for the derivatives dA and dB) in shared
 // memory, then every lane sums the products of its own (component, value) items over
-// the units.  Bound: shared-memory reads of the product step, three per two FP64
+// the units.  The slices of a pair are warps of one block or cluster; their sums meet in
+// shared memory, in order, so that one lane writes V(i,j) and V(j,i): symmetric to the bit
+// and the same on every call.  (A row of dV takes two atomic adds, the nucleus' own and
+// the centres', whose order does not show.)  Bound: shared-memory reads of the product
+// step, three per two FP64
 // operations; the tables a lane would otherwise recompute per component stay in
 // shared memory once per unit.  The Hermite form this replaces kept its E and R tables
 // in local memory, once per component and lane: 16 atoms (n = 180), S, T, V and the
@@ -401,40 +406,111 @@ __device__ __forceinline__ void nai_pair(const OeiArgs& a, const PairInfo& P, in
             __syncwarp();
         }
     }
+    // the slice's sums, for nai_write
 #pragma unroll
-    for (int j = 0; j < NIT; ++j) {
-        const int it = lane + 32 * j, v = it / NC, c = it - v * NC, ia = c / NB, ib = c - ia * NB;
-        if (it >= NC * NV || (same && ib > ia)) continue;
-        const long long i0 = P.bf1 + ia, j0 = P.bf2 + ib;
-        double* o = !DER ? a.V : a.dV + (3LL * (v < 3 ? P.atom1 : P.atom2) + v % 3) * nn;
-        atomicAdd(o + i0 * n + j0, tot[j]);
-        if (i0 != j0) atomicAdd(o + j0 * n + i0, tot[j]);
+    for (int j = 0; j < NIT; ++j)
+        if (lane + 32 * j < NC * NV) sm[lane + 32 * j] = tot[j];
+}
+
+// A pair's sums over its nslice slices (slice s at part(s)), in order, to V or to the rows
+// of its two atoms in dV.
+template <bool DER, class Part>
+__device__ __forceinline__ void nai_write(const OeiArgs& a, const PairInfo& P, int nslice, int lane, Part&& part) {
+    const int nb = ncart_h(P.l2), nc = ncart_h(P.l1) * nb;
+    const bool same = P.s1 == P.s2;
+    const long long n = a.n, nn = n * n;
+    for (int it = lane; it < (DER ? 3 * nc : nc); it += 32) {
+        const int x = it / nc, c = it - x * nc, ia = c / nb, ib = c - ia * nb;
+        if (same && ib > ia) continue;
+        const long long ij = (P.bf1 + ia) * n + P.bf2 + ib, ji = (P.bf2 + ib) * n + P.bf1 + ia;
+        double va = 0.0, vb = 0.0;
+        for (int s = 0; s < nslice; ++s) {
+            const double* q = part(s);
+            va += q[it];
+            if (DER) vb += q[it + 3 * nc];
+        }
+        if constexpr (!DER) {
+            a.V[ij] = va;
+            a.V[ji] = va;
+        } else {
+            auto add = [&](int atom, double v) {
+                double* o = a.dV + (3LL * atom + x) * nn;
+                atomicAdd(o + ij, v);
+                if (ij != ji) atomicAdd(o + ji, v);
+            };
+            if (P.atom1 == P.atom2) {
+                add(P.atom1, va + vb);
+            } else {
+                add(P.atom1, va);
+                add(P.atom2, vb);
+            }
+        }
     }
 }
 
+// wpp warps of each of ncta blocks (a cluster, if more than one; then wpp = 4) share a
+// pair; a slice is `slice` nuclei.
 template <bool DER>
-__global__ void __launch_bounds__(128) k_nai(OeiArgs a, int slice) {
+__global__ void __launch_bounds__(128) k_nai(OeiArgs a, int slice, int wpp, int ncta) {
+    namespace cg = cooperative_groups;
     __shared__ double sm[4][NAI_SM];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int pidx = blockIdx.x * 4 + warp;
-    if (pidx >= a.npair) return;
-    const int lo = blockIdx.y * slice, hi = min(a.natom, lo + slice);
-    const PairInfo P = a.pairs[pidx];
-    switch (P.l1 * (OEI_LMAX + 1) + P.l2) {
-        case 0: return nai_pair<0, 0, DER>(a, P, lo, hi, sm[warp], lane);
-        case 4: return nai_pair<1, 0, DER>(a, P, lo, hi, sm[warp], lane);
-        case 5: return nai_pair<1, 1, DER>(a, P, lo, hi, sm[warp], lane);
-        case 8: return nai_pair<2, 0, DER>(a, P, lo, hi, sm[warp], lane);
-        case 9: return nai_pair<2, 1, DER>(a, P, lo, hi, sm[warp], lane);
-        case 10: return nai_pair<2, 2, DER>(a, P, lo, hi, sm[warp], lane);
-        case 12: return nai_pair<3, 0, DER>(a, P, lo, hi, sm[warp], lane);
-        case 13: return nai_pair<3, 1, DER>(a, P, lo, hi, sm[warp], lane);
-        case 14: return nai_pair<3, 2, DER>(a, P, lo, hi, sm[warp], lane);
-        case 15: return nai_pair<3, 3, DER>(a, P, lo, hi, sm[warp], lane);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rank = blockIdx.x % ncta;
+    const int pidx = blockIdx.x / ncta * (4 / wpp) + warp / wpp;
+    const int sl = rank * wpp + warp % wpp, nslice = wpp * ncta;
+    const int lo = sl * slice, hi = min(a.natom, lo + slice);
+    const bool on = pidx < a.npair;
+    PairInfo P;
+    if (on) {
+        P = a.pairs[pidx];
+        switch (P.l1 * (OEI_LMAX + 1) + P.l2) {
+            case 0: nai_pair<0, 0, DER>(a, P, lo, hi, sm[warp], lane); break;
+            case 4: nai_pair<1, 0, DER>(a, P, lo, hi, sm[warp], lane); break;
+            case 5: nai_pair<1, 1, DER>(a, P, lo, hi, sm[warp], lane); break;
+            case 8: nai_pair<2, 0, DER>(a, P, lo, hi, sm[warp], lane); break;
+            case 9: nai_pair<2, 1, DER>(a, P, lo, hi, sm[warp], lane); break;
+            case 10: nai_pair<2, 2, DER>(a, P, lo, hi, sm[warp], lane); break;
+            case 12: nai_pair<3, 0, DER>(a, P, lo, hi, sm[warp], lane); break;
+            case 13: nai_pair<3, 1, DER>(a, P, lo, hi, sm[warp], lane); break;
+            case 14: nai_pair<3, 2, DER>(a, P, lo, hi, sm[warp], lane); break;
+            case 15: nai_pair<3, 3, DER>(a, P, lo, hi, sm[warp], lane); break;
+        }
     }
+    // every warp of the block, or cluster, to both barriers
+    auto meet = [&] {
+        if (ncta > 1) cg::this_cluster().sync();
+        else if (wpp > 1) __syncthreads();
+        else __syncwarp();
+    };
+    meet();
+    if (on && sl == 0)
+        nai_write<DER>(a, P, nslice, lane, [&](int s) {
+            double* q = sm[warp + s % wpp];  // this is the pair's first warp
+            return (const double*)(s < wpp ? q : cg::this_cluster().map_shared_rank(q, s / wpp));
+        });
+    if (ncta > 1) cg::this_cluster().sync();  // the other blocks' sums are read before they go
 }
 
 }  // namespace qx
+
+template <bool DER>
+static void launch_nai(const qx::OeiArgs& a, cudaStream_t s) {
+    // slices per pair: a power of two, so that they are warps of one block or whole blocks
+    const int want = std::min(a.natom, std::max(1, 148 * 16 / a.npair));
+    int nslice = 1;
+    while (nslice < want && nslice < 32) nslice *= 2;
+    const int wpp = std::min(nslice, 4), ncta = nslice / wpp, ppb = 4 / wpp;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)ncta;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(ncta * ((a.npair + ppb - 1) / ppb)));
+    cfg.blockDim = dim3(128);
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = ncta > 1 ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, qx::k_nai<DER>, a, (a.natom + nslice - 1) / nslice, wpp, ncta);
+}
 
 // Launch over every shell pair of a handle; outputs are zeroed by the caller where
 // derivatives accumulate.  The nuclei are cut into slices until the warps fill the GPU
@@ -463,13 +539,6 @@ void qx_launch_oei(const qx::PairInfo* pairs, int npair, const qx::PrimPair* pri
     if (!blocks) return;
     if (S || T || dS || a.nuc) qx::k_oei<<<blocks, 128, 0, s>>>(a);
     if (a.nuc) return;
-    const int want = std::min(natom, std::max(1, 148 * 16 / npair));
-    const int slice = (natom + want - 1) / want;
-    const dim3 grid(blocks, (natom + slice - 1) / slice);
-    if (dV) {
-        qx::k_nai<true><<<grid, 128, 0, s>>>(a, slice);
-    } else if (V) {
-        cudaMemsetAsync(V, 0, sizeof(double) * n * n, s);
-        qx::k_nai<false><<<grid, 128, 0, s>>>(a, slice);
-    }
+    if (dV) launch_nai<true>(a, s);
+    else if (V) launch_nai<false>(a, s);
 }

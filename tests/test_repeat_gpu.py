@@ -8,6 +8,7 @@ import torch
 
 from quax_b200.basis import Basis, Shell
 from quax_b200.integrals.engine import EriEngine
+from quax_b200.oei import one_electron
 
 pytestmark = pytest.mark.gpu
 
@@ -50,3 +51,28 @@ def test_integrals(ks, engine):
     for p in itertools.permutations(range(4)):
         if {p[0], p[1]} in ({0, 1}, {2, 3}):
             assert bool(((G.permute(p) == G) | own).all()), p
+
+
+# atoms, how many of them carry shells: nuclei in 2, 4, 16 and 32 slices (one to eight
+# blocks per shell pair), some of them empty, and in one slice
+@pytest.mark.parametrize("natom,carry,ls", [(2, 2, (0, 1, 2)), (3, 3, (0, 1, 2)), (12, 4, (0, 1)), (24, 3, (0, 1, 2)),
+                                            (10, 10, (0,) * 5)])
+def test_attraction(natom, carry, ls):
+    """V and dV: every image and every call to the bit (each pair's sums over the nuclei
+    meet in order), and right."""
+    rng = np.random.default_rng(natom)
+    xyz = 1.7 * np.array(list(np.ndindex(3, 3, 3)))[rng.permutation(27)[:natom]] + rng.uniform(-0.2, 0.2, (natom, 3))
+    k = 2 if natom < 10 else 1
+    shells = [Shell(l, rng.uniform(0.2, 20.0, size=k), rng.uniform(0.2, 1.0, size=k), xyz[a], a)
+              for a in range(carry) for l in ls]
+    b = Basis(shells, natom)
+    Z = rng.integers(1, 9, size=natom).astype(float)
+    eng = EriEngine(b, 1e-12)
+    eng.set_charges(Z)
+    V, dV = eng.oei()[2].clone(), eng.oei_deriv(1)[2].clone()
+    assert torch.equal(V, V.T) and torch.equal(dV, dV.transpose(1, 2))
+    for _ in range(5):
+        assert torch.equal(eng.oei()[2], V) and torch.equal(eng.oei_deriv(1)[2], dV)
+    ref = one_electron(b, Z, b.atom_coords(), deriv=True)
+    assert np.abs(V.cpu().numpy() - ref[2]).max() < 1e-12 * max(1.0, np.abs(ref[2]).max())
+    assert np.abs(dV.cpu().numpy() - ref[5]).max() < 1e-11 * max(1.0, np.abs(ref[5]).max())
