@@ -1263,7 +1263,7 @@ static int rys_unsupported(int c, const char* what) {
 }
 
 // Work items that share a quartet's primitives in the Rys kernels: a team walks its
-// primitives one after another (up to 4,096 of them), so few quartets would leave most
+// primitives one after another (thousands of them), so few quartets would leave most
 // of the GPU idle behind the largest one.  The outputs are sums of atomics either way.
 static int rys_parts(long long items, long long max_prims) {
     return (int)std::min(148LL * 32 / items + 1, std::max(1LL, max_prims / 4));

@@ -6,17 +6,26 @@
 
 namespace qx {
 
-constexpr int SEG_POW = 13;  // powers of two a count is compared with: 2^0 .. 2^12
+// Powers of two a count is compared with: 2^0 .. 2^24, the primitives of a quartet of four
+// shells of 64.
+constexpr int SEG_POW = 25;
 
-// Order key of a primitive count.
-inline int seg_key(long long n) { return (int)std::min(n, 4096LL) - 1; }
+// Order key of a primitive count: every count of its own up to 4,096, above in steps of
+// 1/64, none of which spans a power of two.
+inline int seg_key(long long n) {
+    const long long m = std::min(n, 1LL << 24) - 1;
+    if (m < 4096) return (int)m;
+    int e = 12;
+    while (m >> (e + 1)) ++e;
+    return 4096 + (e - 12) * 64 + (int)((m >> (e - 6)) & 63);
+}
 
 // From the histogram over keys 0 .. nkey - 1 (summed over threads already): the quartets
 // with more than 2^k primitives.
 inline void seg_prefix(const long long* hist, int nkey, long long* prefix) {
     for (int k = 0; k < SEG_POW; ++k) {
         long long s = 0;
-        for (int b = 1 << k; b < nkey; ++b) s += hist[b];
+        for (int b = seg_key((1LL << k) + 1); k < 24 && b < nkey; ++b) s += hist[b];
         prefix[k] = s;
     }
 }
@@ -41,7 +50,7 @@ inline int sl_segments(long long nq, long long prims, long long max_prims, const
         return 1;
     }
     const long long threads = 148LL * 768;
-    const long long share = std::min(4096LL, prims < threads ? 16LL : std::max(64LL, prims / threads));
+    const long long share = prims < threads ? 16LL : std::max(64LL, prims / threads);
     int low = 4;
     while (low < SEG_POW - 1 && (2LL << low) <= share) ++low;
     int top = 0;  // lanes of the largest quartets

@@ -43,7 +43,9 @@ def _prefix(seg, counts):
 
 # quartets per primitive count: small, ordinary, and beyond 32 bits in all or in one count
 COUNTS = [{1: 7}, {1: 100, 64: 3}, {1: 5, 3: 5, 9: 5, 27: 5, 81: 5}, {1: 1 << 20, 30: 1 << 18, 4096: 2000},
-          {1: 3 << 30, 8: 1 << 29, 512: 1 << 20}, {16: 5 << 30}, {1: 1 << 31, 4096: (1 << 31) + 5}]
+          {1: 3 << 30, 8: 1 << 29, 512: 1 << 20}, {16: 5 << 30}, {1: 1 << 31, 4096: (1 << 31) + 5},
+          # shells of more than 8 primitives, up to four of 64
+          {1: 300, 4097: 20, 10000: 1000, 1 << 24: 3}, {8: 100, 20736: 4, 20737: 4, 40000: 4}, {1 << 24: 1 << 20}]
 
 
 @pytest.mark.parametrize("ordered", [True, False])
@@ -79,6 +81,17 @@ def test_segments(seg, case, ordered):
             assert (st[j - 1] if j else nb.value) == st[j] + ((hi - f[j]) << j)
             if ordered and hi > f[j]:
                 assert j == ns - 1 and 1 << (j + 1) > cap or largest(f[j], hi) <= share << j
+
+
+def test_keys(seg):
+    """Keys order counts and keep apart those at a power of two; above 4,096 they span at
+    most 1/64 of the count."""
+    ns = sorted({max(1, (1 << k) + d) for k in range(25) for d in (-1, 0, 1)} | set(range(1, 9000, 7)))
+    ns = [n for n in ns if n <= 1 << 24]
+    keys = [seg.seg_key_of(n) for n in ns]
+    assert keys == sorted(keys)
+    for a, b, ka, kb in zip(ns, ns[1:], keys, keys[1:]):
+        assert ka < kb or (b > 4096 and b - a <= b / 64 and (a - 1).bit_length() == (b - 1).bit_length())
 
 
 def test_lanes_by_average(seg):

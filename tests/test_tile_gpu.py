@@ -91,3 +91,31 @@ def test_straight_line_jk(oracle_lib, lg):
         J, K = (x.cpu().numpy() for x in eng.jk(torch.from_numpy(D).cuda(), **kw))
         assert np.abs(J - np.einsum("ijkl,kl->ij", G, D)).max() < 1e-10
         assert np.abs(K - np.einsum("ikjl,kl->ij", G, D)).max() < 1e-10
+
+
+@pytest.mark.parametrize("engine", ["default", "rys"])
+def test_long_contractions(oracle_lib, engine):
+    """Shells of 1, 9 and 12 primitives: quartets of up to 20,736, past the counts that
+    have an order key of their own, in every output that their parts meet in."""
+    rng = np.random.default_rng(23)
+    shells = []
+    for a, x in enumerate(([0.0, 0.0, 0.0], [0.4, -1.1, 1.9])):
+        for l, k in ((0, 12), (1, 9), (1, 12), (2, 1)) if a else ((0, 1), (0, 12), (1, 12)):
+            e = np.sort(np.exp(rng.uniform(np.log(0.2), np.log(20.0), size=k)))[::-1].copy()
+            shells.append(Shell(l, e, rng.uniform(0.2, 1.0, size=k), np.array(x), a))
+    b = Basis(shells, 2)
+    ob = oracle_lib.OracleBasis(b)
+    eng = EriEngine(b, 1e-12)
+    if engine == "rys":
+        for c in eng.class_info():
+            eng.set_engine(c["cls"], plain="rys", deriv="rys")
+    G = oracle_lib.compute_2e_int(ob, 1e-12)
+    assert np.abs(eng.eri().cpu().numpy() - G).max() < 1e-12
+    D = _density(eng.nbf, 6)
+    Dg = torch.from_numpy(D).cuda()
+    J, K = (x.cpu().numpy() for x in eng.jk(Dg))
+    assert np.abs(J - np.einsum("ijkl,kl->ij", G, D)).max() < 1e-10
+    assert np.abs(K - np.einsum("ikjl,kl->ij", G, D)).max() < 1e-10
+    g = eng.grad_adjoint(Dg, 2.0, -1.0).cpu().numpy()
+    gr = oracle_lib.grad_contract(ob, 1e-12, D, 2.0, -1.0)
+    assert np.abs(g - gr).max() < 1e-9 * max(1.0, np.abs(gr).max())
