@@ -24,6 +24,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <string>
 #include <thread>
 #include <vector>
@@ -311,13 +312,6 @@ struct qx_handle {
     double f32_bound = 0.0;  // mixed precision: FP32 recurrences below this Schwarz bound
 };
 
-// Primitive-chunk tasks (quartet, first primitive quartet) of the split modes,
-// built at set-up for the classes that use them by default and otherwise at the
-// first call that needs them; the derivative accumulator buffer is allocated at
-// the first derivative call (need_dacc).  The quartets are cut into slices of at
-// most QX_SPLIT_ACC_BYTES of derivative accumulators; each slice runs as its own
-// VRR + HRR pair.  `list` is the class's current view when the caller has it on
-// the host (set-up), else it is copied back from the device.
 // Runs f(0..nt-1) on nt host threads (f(0) on the caller's).
 template <class F>
 static void host_parallel(int nt, F&& f) {
@@ -327,105 +321,110 @@ static void host_parallel(int nt, F&& f) {
     for (auto& th : pool) th.join();
 }
 
-// Processing order of the classes' views (lists[c] on the host): by primitive quartets,
-// largest first, stable.  The list itself keeps the order of the contracted primitive
-// counts (the unique layout); once negligible primitive pairs are dropped, neighbours
-// there differ several-fold in work, and a straight-line kernel's warp takes as long as
-// its longest lane.  A class of equal counts needs none, and one of more than 2^31 - 1
-// quartets, whose positions the order's entries do not hold, runs in list order.
-static int build_orders(qx_handle* h, const int2* const* lists) {
-    cudaFree(h->d_orders);
-    h->d_orders = nullptr;
-    // keys up to the largest quartet of the handle
+// Processing order of the classes' views: by primitive quartets, largest first, stable.
+// The list itself keeps the order of the contracted primitive counts (the unique layout);
+// once negligible primitive pairs are dropped, neighbours there differ several-fold in
+// work, and a straight-line kernel's warp takes as long as its longest lane.  A class of
+// equal counts needs none.  The order is not needed for the results: a class of more than
+// 2^31 - 1 quartets, whose positions the entries do not hold, and a device or host without
+// room for the entries (half of the quartet list) run in list order.
+//
+// A counting sort over host threads, in two steps so that one class's list is on the host
+// at a time: thread t counts its contiguous range (count_order, which leaves every
+// thread's first position per key in `pos`), and writes it (write_orders).
+static int order_threads(long long nq) {
+    return (int)std::max<long long>(1, std::min<long long>({16, (long long)std::thread::hardware_concurrency(),
+                                                            nq / 16384}));
+}
+static long long quartet_prims(const qx_handle* h, const int2& q) {
+    return (long long)h->pairs[q.x].nprim * h->pairs[q.y].nprim;
+}
+static int order_keys(const qx_handle* h) {  // up to the largest quartet of the handle
     int pmax = 1;
     for (const auto& p : h->pairs) pmax = std::max(pmax, p.nprim);
-    const int NB = seg_key((long long)pmax * pmax) + 1;
-    long long total = 0, work = 0;
-    std::vector<long long> off(QX_NCLS_ALL, 0);
-    std::vector<int> live;
-    for (int c = 0; c < QX_NCLS_ALL; ++c) {
-        ClassWork& w = h->work[c];
-        w.d_order = nullptr;
-        off[c] = total;
-        if (!w.nq) continue;
-        live.push_back(c);
-        work += w.nq;
-        if (w.nq <= 0x7fffffffLL) total += w.nq;
+    return seg_key((long long)pmax * pmax) + 1;
+}
+
+static void count_order(qx_handle* h, int c, const int2* list, int nkey, std::vector<long long>& pos) {
+    ClassWork& w = h->work[c];
+    w.d_order = nullptr;
+    w.uniform = true;
+    w.max_prims = 0;
+    if (!w.nq) return;
+    const int nt = order_threads(w.nq);
+    pos.assign((size_t)nt * nkey, 0);
+    std::vector<long long> top(nt, 0), sum(nkey, 0);
+    host_parallel(nt, [&](int t) {
+        long long* H = pos.data() + (size_t)t * nkey;
+        for (long long q = w.nq * t / nt; q < w.nq * (t + 1) / nt; ++q) {
+            const long long n = quartet_prims(h, list[q]);
+            ++H[seg_key(n)];
+            top[t] = std::max(top[t], n);
+        }
+    });
+    long long run = 0;
+    int used = 0;
+    for (int b = nkey - 1; b >= 0; --b) {  // largest first
+        const long long before = run;
+        for (int t = 0; t < nt; ++t) {
+            long long& x = pos[(size_t)t * nkey + b];
+            const long long v = x;
+            x = run;
+            run += v;
+        }
+        sum[b] = run - before;
+        used += run != before;
     }
-    std::unique_ptr<int[]> order(new int[(size_t)std::max(1LL, total)]);
-    // a counting sort over host threads: thread t counts its contiguous range of every
-    // class, and after a scan in (key, thread) order writes it
-    const int nt = (int)std::max<long long>(1, std::min<long long>({16, (long long)std::thread::hardware_concurrency(),
-                                                                    work / 16384}));
-    const size_t nl = live.size();
-    std::vector<std::vector<long long>> hist(nt);
-    auto prims = [&](const int2& q) { return (long long)h->pairs[q.x].nprim * h->pairs[q.y].nprim; };
-    auto key = [&](const int2& q) { return NB - 1 - seg_key(prims(q)); };  // largest first
-    host_parallel(nt, [&](int t) {
-        hist[t].assign(nl * NB, 0);
-        for (size_t k = 0; k < nl; ++k) {
-            const long long nq = h->work[live[k]].nq;
-            long long* H = hist[t].data() + k * NB;
-            for (long long q = nq * t / nt; q < nq * (t + 1) / nt; ++q) ++H[key(lists[live[k]][q])];
+    w.uniform = used == 1;
+    w.max_prims = *std::max_element(top.begin(), top.end());
+    seg_prefix(sum.data(), nkey, w.prefix);
+    if (w.uniform || w.nq > 0x7fffffffLL) std::vector<long long>().swap(pos);
+}
+
+// list(c): class c's view on the host, valid until the next call.
+template <class List>
+static int write_orders(qx_handle* h, int nkey, std::vector<long long>* pos, List&& list) {
+    cudaFree(h->d_orders);
+    h->d_orders = nullptr;
+    long long total = 0, most = 0;
+    for (int c = 0; c < QX_NCLS_ALL; ++c)
+        if (!pos[c].empty()) {
+            total += h->work[c].nq;
+            most = std::max(most, h->work[c].nq);
         }
-    });
-    host_parallel(nt, [&](int t) {
-        std::vector<long long> sum(NB);
-        for (size_t k = t; k < nl; k += nt) {
-            ClassWork& w = h->work[live[k]];
-            long long run = 0;
-            int used = 0;
-            for (int b = 0; b < NB; ++b) {
-                const long long before = run;
-                for (int u = 0; u < nt; ++u) {
-                    long long& x = hist[u][k * NB + b];
-                    const long long v = x;
-                    x = run;
-                    run += v;
-                }
-                sum[NB - 1 - b] = run - before;
-                used += run != before;
-            }
-            w.uniform = used == 1;
-            seg_prefix(sum.data(), NB, w.prefix);
-        }
-    });
-    std::vector<long long> top((size_t)nt * nl, 0);
-    host_parallel(nt, [&](int t) {
-        for (size_t k = 0; k < nl; ++k) {
-            const int c = live[k];
-            const ClassWork& w = h->work[c];
-            const long long nq = w.nq;
-            const bool sort = !w.uniform && nq <= 0x7fffffffLL;
-            long long* H = hist[t].data() + k * NB;
-            int* o = order.get() + off[c];
-            long long mx = 0;
-            for (long long q = nq * t / nt; q < nq * (t + 1) / nt; ++q) {
-                mx = std::max(mx, prims(lists[c][q]));
-                if (sort) o[H[key(lists[c][q])]++] = (int)q;
-            }
-            top[(size_t)t * nl + k] = mx;
-        }
-    });
-    bool any = false;
-    for (size_t k = 0; k < nl; ++k) {
-        ClassWork& w = h->work[live[k]];
-        w.max_prims = 0;
-        for (int t = 0; t < nt; ++t) w.max_prims = std::max(w.max_prims, top[(size_t)t * nl + k]);
-        any = any || (!w.uniform && w.nq <= 0x7fffffffLL);
-    }
-    if (!any) return QX_OK;
-    if (cudaMalloc((void**)&h->d_orders, sizeof(int) * total) != cudaSuccess) {
+    if (!total) return QX_OK;
+    std::unique_ptr<int[]> order(new (std::nothrow) int[(size_t)most]);
+    if (!order || cudaMalloc((void**)&h->d_orders, sizeof(int) * total) != cudaSuccess) {
         cudaGetLastError();
         h->d_orders = nullptr;
-        return fail(QX_E_NOMEM, "processing order of %lld quartets", total);
+        return QX_OK;  // list order
     }
-    QX_CUDA(cudaMemcpy(h->d_orders, order.get(), sizeof(int) * total, cudaMemcpyHostToDevice));
-    for (int c : live)
-        if (!h->work[c].uniform && h->work[c].nq <= 0x7fffffffLL) h->work[c].d_order = h->d_orders + off[c];
+    long long off = 0;
+    for (int c = 0; c < QX_NCLS_ALL; ++c) {
+        if (pos[c].empty()) continue;
+        ClassWork& w = h->work[c];
+        const int2* L = list(c);
+        if (!L) return fail(QX_E_CUDA, "quartet list of a class not read back");
+        const int nt = order_threads(w.nq);
+        host_parallel(nt, [&](int t) {
+            long long* H = pos[c].data() + (size_t)t * nkey;
+            for (long long q = w.nq * t / nt; q < w.nq * (t + 1) / nt; ++q)
+                order[H[seg_key(quartet_prims(h, L[q]))]++] = (int)q;
+        });
+        QX_CUDA(cudaMemcpy(h->d_orders + off, order.get(), sizeof(int) * w.nq, cudaMemcpyHostToDevice));
+        w.d_order = h->d_orders + off;
+        off += w.nq;
+    }
     return QX_OK;
 }
 
+// Primitive-chunk tasks (quartet, first primitive quartet) of the split modes,
+// built at set-up for the classes that use them by default and otherwise at the
+// first call that needs them; the derivative accumulator buffer is allocated at
+// the first derivative call (need_dacc).  The quartets are cut into slices of at
+// most QX_SPLIT_ACC_BYTES of derivative accumulators; each slice runs as its own
+// VRR + HRR pair.  `list` is the class's current view when the caller has it on
+// the host (set-up), else it is copied back from the device.
 static int ensure_split_tasks(qx_handle* h, int c, bool need_dacc = false, const int2* list = nullptr,
                               bool sync = true) {
     ClassWork& w = h->work[c];
@@ -937,9 +936,10 @@ extern "C" int qx_initialize(int natom, const double* coords, int nshell, const 
     std::sort(h->order, h->order + QX_NCLS_ALL,
               [&](int x, int y) { return full_c[x] * g_class_nout[x] > full_c[y] * g_class_nout[y]; });
     {
-        const int2* lists[QX_NCLS_ALL];
-        for (int c = 0; c < QX_NCLS_ALL; ++c) lists[c] = sorted[c].get();
-        const int rc = build_orders(h, lists);
+        const int nkey = order_keys(h);
+        std::vector<long long> pos[QX_NCLS_ALL];
+        for (int c = 0; c < QX_NCLS_ALL; ++c) count_order(h, c, sorted[c].get(), nkey, pos[c]);
+        const int rc = write_orders(h, nkey, pos, [&](int c) { return (const int2*)sorted[c].get(); });
         if (rc) {
             free_handle(h);
             return rc;
@@ -1000,8 +1000,9 @@ extern "C" int qx_partition_costs(const double* cost, long long n, int nranks, l
 static int rebuild_views(qx_handle* h) {
     QX_CUDA(cudaDeviceSynchronize());
     const int rank = h->shard_rank, nranks = h->shard_n;
-    std::vector<std::vector<int2>> full(QX_NCLS_ALL);
-    const int2* lists[QX_NCLS_ALL];
+    const int nkey = order_keys(h);
+    std::vector<long long> pos[QX_NCLS_ALL];
+    std::vector<int2> L;
     long long base = 0;
     h->nunique = 0;
     for (int c = 0; c < QX_NCLS_ALL; ++c) {
@@ -1016,9 +1017,8 @@ static int rebuild_views(qx_handle* h) {
         w.slice_t.clear();
         long long lo = 0, hi = w.nq_full;
         long long prims = 0;
-        std::vector<int2>& L = full[c];
-        L.resize((size_t)w.nq_full);
         if (w.nq_full) {
+            L.resize((size_t)w.nq_full);
             QX_CUDA(cudaMemcpy(L.data(), w.d_q_full, sizeof(int2) * w.nq_full, cudaMemcpyDeviceToHost));
             std::vector<double> cost((size_t)w.nq_full);
             for (long long i = 0; i < w.nq_full; ++i)
@@ -1037,10 +1037,15 @@ static int rebuild_views(qx_handle* h) {
         w.unique_base = base;
         base += w.nq * g_class_nout[c];
         h->nunique += w.nq;
-        lists[c] = L.data() + lo;
+        count_order(h, c, L.data() + lo, nkey, pos[c]);
     }
     h->unique_size = base;
-    int rc = build_orders(h, lists);
+    const int rc = write_orders(h, nkey, pos, [&](int c) -> const int2* {
+        const ClassWork& w = h->work[c];
+        L.resize((size_t)w.nq);
+        return cudaMemcpy(L.data(), w.d_q, sizeof(int2) * w.nq, cudaMemcpyDeviceToHost) == cudaSuccess ? L.data()
+                                                                                                      : nullptr;
+    });
     if (rc) return rc;
     QX_CUDA(cudaDeviceSynchronize());  // the order lists have landed before any stream reads them
     return QX_OK;

@@ -80,3 +80,38 @@ def test_layout_of_views():
     assert sorted(got) == sorted(ref)
     for k, v in got.items():
         assert np.abs(v - ref[k]).max() <= 1e-13 * max(1.0, np.abs(ref[k]).max()), k
+
+
+def test_order_without_room():
+    """A device with room for the quartet lists but not for their processing order: the
+    handle works, in list order."""
+    rng = np.random.default_rng(31)
+    xyz = 1.6 * np.array(list(np.ndindex(5, 5, 5)))[:110] + rng.uniform(-0.2, 0.2, (110, 3))
+    shells = [Shell(0, rng.uniform(0.08, 0.4, size=1 + a % 3), np.ones(1 + a % 3), xyz[a], a) for a in range(110)]
+    b = Basis(shells, 110)
+
+    def free():
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        return torch.cuda.mem_get_info()[0]
+
+    D = torch.eye(110, dtype=torch.float64, device="cuda")
+    warm = EriEngine(b, 1e-12)  # what the first calls of a process allocate
+    warm.jk(D)
+    warm.close()
+    f0 = free()
+    ref = EriEngine(b, 1e-12)
+    used = f0 - free()
+    nq = ref.unique_quartets()
+    assert used > 12 * nq > 100 << 20  # lists of 8 bytes and orders of 4 per quartet
+    J, K = ref.jk(D)
+    ref.close()
+    fill = torch.empty(free() - used + 2 * nq, dtype=torch.uint8, device="cuda")
+    eng = EriEngine(b, 1e-12)
+    J2, K2 = eng.jk(D)
+    eng.set_precision(1e-9)  # lists rebuilt, with no more room than before
+    eng.set_precision(0.0)
+    J3, K3 = eng.jk(D)
+    del fill
+    for x, y in ((J, J2), (K, K2), (J, J3), (K, K3)):
+        assert (x - y).abs().max().item() < 1e-11 * J.abs().max().item()
