@@ -219,12 +219,13 @@ int qx_autotune(qx_handle *h, int what, void *stream);
 
 /* Engine configuration of one class: cfg[0] plain engine (0 straight-line,
  * 1 warp, 2 cooperative, 4 warp VRR into global accumulators + warp HRR, 6 Rys
- * quadrature), cfg[1] its parameter (log2 lanes per quartet, or warps per quartet;
- * straight-line kernels left to themselves choose the lanes by the quartet's
- * primitives), cfg[2] engine of the adjoint gradient (1 warp, 2 cooperative, 3 warp
- * VRR into global accumulators + cooperative HRR, 5 warp VRR into global
- * accumulators + warp HRR, 6 Rys), cfg[3] its warps per quartet (Rys: the parameter
- * qx_set_engine was given). */
+ * quadrature), cfg[1] its parameter (log2 lanes per quartet, -1 where a straight-line
+ * kernel chooses them by the quartet's primitives; or warps per quartet), cfg[2] engine of
+ * the adjoint gradient (1 warp, 2 cooperative, 3 warp VRR into global accumulators +
+ * cooperative HRR, 5 warp VRR into global accumulators + warp HRR, 6 Rys), cfg[3] its
+ * parameter: warps per quartet; for Rys the one qx_set_engine was given, or, where the
+ * first-derivative tensors run on another engine, 8 * that engine + its warps per quartet
+ * (0 if it takes none).  qx_set_engine with these four values restores the choice. */
 int qx_engine_config(const qx_handle *h, int cls, int *cfg);
 
 /* Engine of one class chosen by the caller, no counterpart in the reference: the
@@ -232,8 +233,8 @@ int qx_engine_config(const qx_handle *h, int cls, int *cfg);
  * engine ids as qx_engine_config reports them (6 = Rys quadrature, available for
  * every class), -1 keeps the current choice; pparam / dparam as in
  * qx_engine_config (Rys derivative engine: 0 or 1, the same program).  deriv sets the
- * engine of the adjoint gradient and of the first-derivative tensors.  QX_E_UNSUPPORTED when the class lacks the engine.
- * Synchronises the device. */
+ * engine of the adjoint gradient and, unless dparam names another, of the first-derivative
+ * tensors.  QX_E_UNSUPPORTED when the class lacks the engine.  Synchronises the device. */
 int qx_set_engine(qx_handle *h, int cls, int plain, int pparam, int deriv, int dparam);
 
 /* Bounded waits, no counterpart in the reference: the split-mode kernels stage

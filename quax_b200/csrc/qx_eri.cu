@@ -1862,8 +1862,10 @@ extern "C" int qx_autotune(qx_handle* h, int what, void* stream) {
 // Engine of one class chosen by the caller (tests, measurements): the autotuner's
 // choice made by hand.  plain / deriv: engine ids as qx_engine_config reports
 // them, -1 keeps the current one; pparam / dparam: log2 lanes per quartet
-// (straight-line) or warps per quartet (warp kernels); the Rys derivative engine
-// takes dparam 0 or 1, which select the same program; ignored otherwise.
+// (straight-line; -1 = by the quartet's primitives) or warps per quartet (warp kernels);
+// the Rys derivative engine takes dparam 0 or 1, which select the same program, or
+// 8 * engine + warps per quartet for first-derivative tensors of another engine; ignored
+// otherwise.  What qx_engine_config reports restores the engines it was asked about.
 extern "C" int qx_set_engine(qx_handle* h, int cls, int plain, int pparam, int deriv, int dparam) {
     if (!h || cls < 0 || cls >= QX_NCLS_ALL) return fail(QX_E_INVALID, "qx_set_engine: bad handle or class");
     DeviceGuard g(h->device);
@@ -1875,7 +1877,7 @@ extern "C" int qx_set_engine(qx_handle* h, int cls, int plain, int pparam, int d
     };
     if (plain >= 0) {
         bool ok = false;
-        if (plain == ENG_SL) ok = has_os(cls) && !g_class_coop[cls] && pparam >= 0 && pparam <= 5;
+        if (plain == ENG_SL) ok = has_os(cls) && !g_class_coop[cls] && pparam >= -1 && pparam <= 5;
         if (plain == ENG_WARP) ok = has_os(cls) && g_has_warp_plain[cls] && (pparam == 1 || pparam == 4);
         if (plain == ENG_COOP) ok = has_os(cls) && g_class_coop[cls];
         if (plain == ENG_WSPLIT) ok = has_os(cls) && g_has_pvrr[cls] && g_has_warp_plain[cls];
@@ -1885,7 +1887,7 @@ extern "C" int qx_set_engine(qx_handle* h, int cls, int plain, int pparam, int d
         if (plain == ENG_SL && g_class_scratch[cls] && w.nq) {  // global accumulators for this lane count
             cudaFree(w.scratch);
             w.scratch = nullptr;
-            if (cudaMalloc((void**)&w.scratch, sizeof(double) * g_class_scratch[cls] * launch_threads(w.nq, pparam)) !=
+            if (cudaMalloc((void**)&w.scratch, sizeof(double) * g_class_scratch[cls] * launch_threads(w.nq, std::max(0, pparam))) !=
                 cudaSuccess) {
                 cudaGetLastError();
                 w.scratch = nullptr;
@@ -1898,23 +1900,28 @@ extern "C" int qx_set_engine(qx_handle* h, int cls, int plain, int pparam, int d
         }
         h->plain_eng[cls] = plain;
         if (plain == ENG_SL) {
-            w.log2g = pparam;
-            w.sl_auto = false;
+            w.sl_auto = pparam < 0;
+            if (pparam >= 0) w.log2g = pparam;
         }
         if (plain == ENG_WARP) h->wpq[cls] = pparam;
         if (plain == ENG_WSPLIT) h->wpq[cls] = 1;
     }
     if (deriv >= 0) {
+        // the engine of the first-derivative tensors: the gradient's, unless that is Rys and
+        // dparam names another one
+        const int te = deriv == ENG_RYS && dparam >= 8 ? dparam / 8 : deriv;
+        const int tp = te == deriv ? dparam : dparam % 8;
         bool ok = false;
-        if (deriv == ENG_WARP) ok = has_os(cls) && g_has_warp_deriv[cls] && (dparam == 1 || dparam == 4);
-        if (deriv == ENG_WVRR) ok = has_os(cls) && g_has_wvrr[cls];
-        if (deriv == ENG_DSPLIT) ok = has_os(cls) && g_has_dsplit[cls];
-        if (deriv == ENG_COOP) ok = g_der_idx[cls] >= 0;
-        if (deriv == ENG_RYS) ok = dparam == 0 || dparam == 1;
-        if (!ok) return no("derivative", deriv);
-        h->deriv_eng[cls] = h->grad_eng[cls] = deriv;
-        if (deriv == ENG_WARP) h->wpq_deriv[cls] = dparam;
-        if (deriv == ENG_RYS) h->rys_param[cls] = dparam;
+        if (te == ENG_WARP) ok = has_os(cls) && g_has_warp_deriv[cls] && (tp == 1 || tp == 4);
+        if (te == ENG_WVRR) ok = has_os(cls) && g_has_wvrr[cls];
+        if (te == ENG_DSPLIT) ok = has_os(cls) && g_has_dsplit[cls];
+        if (te == ENG_COOP) ok = g_der_idx[cls] >= 0;
+        if (te == ENG_RYS) ok = tp == 0 || tp == 1;
+        if (!ok) return no("derivative", te);
+        h->grad_eng[cls] = deriv;
+        h->deriv_eng[cls] = te;
+        if (te == ENG_WARP) h->wpq_deriv[cls] = tp;
+        if (te == ENG_RYS) h->rys_param[cls] = tp;
     }
     return QX_OK;
 }
@@ -1965,9 +1972,12 @@ extern "C" int qx_class_quartets(const qx_handle* h, int cls, int* shells) {
 extern "C" int qx_engine_config(const qx_handle* h, int cls, int* cfg) {
     if (!h || !cfg || cls < 0 || cls >= QX_NCLS_ALL) return fail(QX_E_INVALID, "qx_engine_config: bad argument");
     cfg[0] = h->plain_eng[cls];
-    cfg[1] = h->plain_eng[cls] == ENG_SL ? h->work[cls].log2g : (h->plain_eng[cls] == ENG_WARP ? h->wpq[cls] : 0);
+    const ClassWork& w = h->work[cls];
+    cfg[1] = h->plain_eng[cls] == ENG_SL ? (w.sl_auto ? -1 : w.log2g) : (h->plain_eng[cls] == ENG_WARP ? h->wpq[cls] : 0);
     cfg[2] = h->grad_eng[cls];
-    cfg[3] = h->grad_eng[cls] == ENG_WARP ? h->wpq_deriv[cls] : (h->grad_eng[cls] == ENG_RYS ? h->rys_param[cls] : 0);
+    const int te = h->deriv_eng[cls];
+    if (cfg[2] == ENG_RYS) cfg[3] = te == ENG_RYS ? h->rys_param[cls] : 8 * te + (te == ENG_WARP ? h->wpq_deriv[cls] : 0);
+    else cfg[3] = cfg[2] == ENG_WARP ? h->wpq_deriv[cls] : 0;  // the tensors' engine too
     return QX_OK;
 }
 

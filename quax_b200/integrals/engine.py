@@ -197,7 +197,8 @@ class EriEngine:
             _lib.check(_lib.load().qx_autotune(self.handle, what, C.c_void_p(_stream_ptr(stream))), "qx_autotune")
 
     def engine_config(self):
-        """{"la lb lc ld": (plain engine, param, deriv engine, param)} for the classes with quartets."""
+        """{"la lb lc ld": (plain engine, param, gradient engine, param)} for the classes with
+        quartets; set_engine with these values restores the choice."""
         lib = _lib.load()
         out = {}
         for c in self.class_info():
@@ -211,9 +212,10 @@ class EriEngine:
     def set_engine(self, cls: int, plain: str | None = None, plain_param: int = 0, deriv: str | None = None,
                    deriv_param: int = 0) -> None:
         """Force the engine of one class (names as in ENGINE_NAMES; None keeps the
-        current one).  plain_param: log2 lanes per quartet ("sl") or warps per
-        quartet ("warp": 1 or 4); deriv_param: warps per quartet ("warp"), or 0 or 1
-        for "rys" (the same program)."""
+        current one).  plain_param: log2 lanes per quartet ("sl"; -1 by its primitives) or
+        warps per quartet ("warp": 1 or 4); deriv_param: warps per quartet ("warp"), or for
+        "rys" 0 or 1 (the same program), or 8 * engine + warps per quartet for
+        first-derivative tensors of another engine."""
         pe = -1 if plain is None else self.ENGINE_NAMES.index(plain)
         de = -1 if deriv is None else self.ENGINE_NAMES.index(deriv)
         with torch.cuda.device(self.device):

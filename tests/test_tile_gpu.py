@@ -119,3 +119,42 @@ def test_long_contractions(oracle_lib, engine):
     g = eng.grad_adjoint(Dg, 2.0, -1.0).cpu().numpy()
     gr = oracle_lib.grad_contract(ob, 1e-12, D, 2.0, -1.0)
     assert np.abs(g - gr).max() < 1e-9 * max(1.0, np.abs(gr).max())
+
+
+def test_engine_config_round_trip():
+    """What engine_config reports, given back to set_engine, changes nothing: the lanes a
+    straight-line kernel chooses itself, and tensors on another engine than the gradient."""
+    b = synthetic_molecule(SyntheticSpec(natom=3, box=5.0, min_sep=1.2, kmax=3, exp_lo=0.1, exp_hi=50.0, f_shell=True,
+                                         f_kmax=1), 5)[1]
+    eng = EriEngine(b, 1e-12)
+    classes = {"%d%d%d%d" % c["l"]: c["cls"] for c in eng.class_info() if c["nq"]}
+    names = EriEngine.ENGINE_NAMES
+
+    def apply(cfg):
+        for k, (plain, p, deriv, d) in cfg.items():
+            eng.set_engine(classes[k], plain=plain, plain_param=p, deriv=deriv, deriv_param=d)
+
+    default = eng.engine_config()
+    assert all(v[1] == -1 for v in default.values() if v[0] == "sl")
+    # the tiles' gradient from L = 4 on; tensors of the classes up to d stay on their engine
+    for k, v in default.items():
+        if v[2] == "rys":
+            assert (v[3] in (0, 1)) == ("3" in k)
+            assert "3" in k or names[v[3] // 8] in ("warp", "coop", "wvrr", "dsplit")
+    apply(default)
+    assert eng.engine_config() == default
+    for lg in (0, 5):  # fixed lanes, and tensors and gradient on one engine
+        apply({k: (v[0], lg if v[0] == "sl" else v[1], "rys", 0) for k, v in default.items()})
+        fixed = eng.engine_config()
+        assert all(v[2:] == ("rys", 0) and (v[0] != "sl" or v[1] == lg) for v in fixed.values())
+        apply(fixed)
+        assert eng.engine_config() == fixed
+    apply(default)
+    assert eng.engine_config() == default
+    eng.autotune()
+    tuned = eng.engine_config()
+    apply(tuned)
+    assert eng.engine_config() == tuned
+    for plain_param, deriv_param in ((-2, 0), (6, 0), (-1, 2), (-1, 48), (-1, 8 + 2)):
+        with pytest.raises(NotImplementedError):
+            eng.set_engine(classes["1010"], plain="sl", plain_param=plain_param, deriv="rys", deriv_param=deriv_param)
