@@ -201,10 +201,9 @@ __global__ void __launch_bounds__(AccPolicy<EriCls<LA, LB, LC, LD>::NACC>::bs) k
     using C = EriCls<LA, LB, LC, LD>;
     using Pol = AccPolicy<C::NACC>;
     const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    long long qi = gt >> a.log2g;
+    const long long qi = gt >> a.log2g;
     const int sub = (int)(gt & ((1 << a.log2g) - 1));
     const bool active = qi < a.nq;
-    if (active) qi = list_index(a, qi);
     // every lane stays to the end: the group reduction shuffles over the full warp
     const int2 pq = active ? a.quartets[qi] : make_int2(0, 0);
     const PairInfo P = a.pairs[pq.x];
@@ -226,6 +225,8 @@ __global__ void __launch_bounds__(AccPolicy<EriCls<LA, LB, LC, LD>::NACC>::bs) k
     }
 }
 
+// The non-allocating path's modes: the dense tensor and the Schwarz values (a handle's
+// quartets run in qx_sl.cuh).
 template <int LA, int LB, int LC, int LD>
 void launch_eri(const EriArgs& a, int mode, cudaStream_t s) {
     using Pol = AccPolicy<EriCls<LA, LB, LC, LD>::NACC>;
@@ -236,11 +237,8 @@ void launch_eri(const EriArgs& a, int mode, cudaStream_t s) {
         auto k = k_eri<LA, LB, LC, LD, MODE_DENSE>;
         if (Pol::smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, Pol::smem);
         k<<<(unsigned)nb, bs, Pol::smem, s>>>(a);
-    } else if (mode == MODE_UNIQUE) {
-        auto k = k_eri<LA, LB, LC, LD, MODE_UNIQUE>;
-        if (Pol::smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, Pol::smem);
-        k<<<(unsigned)nb, bs, Pol::smem, s>>>(a);
     } else if constexpr (LA == LC && LB == LD) {
+        if (mode != MODE_SCHWARZ) return;
         auto k = k_eri<LA, LB, LC, LD, MODE_SCHWARZ>;
         if (Pol::smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, Pol::smem);
         k<<<(unsigned)nb, bs, Pol::smem, s>>>(a);
