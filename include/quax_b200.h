@@ -200,11 +200,13 @@ int qx_partition_costs(const double *cost, long long n, int nranks, long long *b
  * whose HRR has at most two transfer steps (lb + ld <= 2: the HRR amplifies the
  * FP32 error about tenfold per step, so the others stay FP64); the primitive
  * set-up, the Boys function, the sums over primitives, the HRR, the epilogues and
- * every accumulation into J, K, gradients and tensors stay FP64.  Each class's
- * list is reordered with its FP64 quartets first, which reorders the unique
- * layout.  bound <= 0 (the default) keeps everything FP64.  Synchronises the
- * device; call qx_autotune afterwards.  qx_precision_split returns how many of a
- * class's quartets (in this rank's view) stay FP64. */
+ * every accumulation into J, K, gradients and tensors stay FP64.  The straight-line,
+ * cooperative and Rys engines keep every quartet FP64; by default that includes the
+ * adjoint gradient of the classes with la + lb + lc + ld >= 4.  Each class's list is reordered
+ * with its FP64 quartets first, which reorders the unique layout.  bound <= 0 (the
+ * default) keeps everything FP64.  Synchronises the device; call qx_autotune
+ * afterwards.  qx_precision_split returns how many of a class's quartets (in this rank's
+ * view) stay FP64 whatever the engine. */
 int qx_set_precision(qx_handle *h, double bound);
 long long qx_precision_split(const qx_handle *h, int cls);
 

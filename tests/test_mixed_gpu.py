@@ -66,3 +66,40 @@ def test_mixed_unique_layout_and_errors():
     assert torch.isfinite(out).all()
     with pytest.raises(ValueError):
         e.set_precision(float("nan"))
+
+
+@pytest.mark.parametrize("engine,param", [("warp", 1), ("warp", 4), ("dsplit", 0), ("wvrr", 0), ("rys", 0)])
+def test_mixed_gradient_engines(engine, param):
+    """The engines with FP32 recurrences run them in the gradient of every class that
+    splits, the default choice aside; the Rys kernels keep FP64."""
+    from quax_b200.integrals.engine import EriEngine
+
+    bound = 1e-6
+    e = EriEngine(_basis(1), 1e-12)
+    n = e.nbf
+    C = np.random.default_rng(2).normal(0.0, 1.0 / np.sqrt(n), size=(n, max(1, n // 4)))
+    D = torch.from_numpy(C @ C.T).cuda()
+    on = []
+    for c in e.class_info():
+        try:
+            e.set_engine(c["cls"], deriv=engine, deriv_param=param)
+            on.append(c)
+        except NotImplementedError:
+            pass
+
+    def grads():
+        return {"%d%d%d%d" % c["l"]: e.grad_adjoint_class(c["cls"], D, torch.zeros(3 * e.natom, dtype=torch.float64,
+                                                                                   device="cuda")) for c in on}
+
+    ref = grads()
+    e.set_precision(bound)
+    split, got = e.precision_split(), grads()
+    fp32 = {k for k, v in split.items() if v[0] < v[1] and k in ref}
+    assert any(sum(map(int, k)) >= 4 for k in fp32)
+    moved = set()
+    for k in ref:
+        d, noise = (got[k] - ref[k]).abs().max().item(), 1e-13 * max(1.0, ref[k].abs().max().item())
+        assert d <= (1e3 * 5e-3 * bound if k in fp32 and engine != "rys" else noise), k
+        if d > noise:
+            moved.add(k)
+    assert (engine == "rys") == (not any(sum(map(int, k)) >= 4 for k in moved))
