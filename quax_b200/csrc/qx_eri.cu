@@ -333,19 +333,27 @@ static void host_parallel(int nt, F&& f) {
 // at a time: thread t counts its contiguous range (count_order, which leaves every
 // thread's first position per key in `pos`), and writes it (write_orders).
 static int order_threads(long long nq) {
-    return (int)std::max<long long>(1, std::min<long long>({16, (long long)std::thread::hardware_concurrency(),
+    return (int)std::max<long long>(1, std::min<long long>({32, (long long)std::thread::hardware_concurrency(),
                                                             nq / 16384}));
 }
-static long long quartet_prims(const qx_handle* h, const int2& q) {
-    return (long long)h->pairs[q.x].nprim * h->pairs[q.y].nprim;
-}
-static int order_keys(const qx_handle* h) {  // up to the largest quartet of the handle
-    int pmax = 1;
-    for (const auto& p : h->pairs) pmax = std::max(pmax, p.nprim);
-    return seg_key((long long)pmax * pmax) + 1;
-}
+struct OrderCounts {
+    std::vector<int> nleft;  // primitive pairs per shell pair, apart from the records: the sort's only reads
+    int nkey = 0;            // keys up to the largest quartet of the handle
+    std::vector<long long> pos[QX_NCLS_ALL];
+    explicit OrderCounts(const qx_handle* h) {
+        int top = 1;
+        for (const auto& p : h->pairs) {
+            nleft.push_back(p.nprim);
+            top = std::max(top, p.nprim);
+        }
+        nkey = seg_key((long long)top * top) + 1;
+    }
+    long long prims(const int2& q) const { return (long long)nleft[q.x] * nleft[q.y]; }
+};
 
-static void count_order(qx_handle* h, int c, const int2* list, int nkey, std::vector<long long>& pos) {
+static void count_order(qx_handle* h, int c, const int2* list, OrderCounts& oc) {
+    const int nkey = oc.nkey;
+    std::vector<long long>& pos = oc.pos[c];
     ClassWork& w = h->work[c];
     w.d_order = nullptr;
     w.uniform = true;
@@ -356,11 +364,13 @@ static void count_order(qx_handle* h, int c, const int2* list, int nkey, std::ve
     std::vector<long long> top(nt, 0), sum(nkey, 0);
     host_parallel(nt, [&](int t) {
         long long* H = pos.data() + (size_t)t * nkey;
+        long long mx = 0;
         for (long long q = w.nq * t / nt; q < w.nq * (t + 1) / nt; ++q) {
-            const long long n = quartet_prims(h, list[q]);
+            const long long n = oc.prims(list[q]);
             ++H[seg_key(n)];
-            top[t] = std::max(top[t], n);
+            mx = std::max(mx, n);
         }
+        top[t] = mx;
     });
     long long run = 0;
     int used = 0;
@@ -383,7 +393,8 @@ static void count_order(qx_handle* h, int c, const int2* list, int nkey, std::ve
 
 // list(c): class c's view on the host, valid until the next call.
 template <class List>
-static int write_orders(qx_handle* h, int nkey, std::vector<long long>* pos, List&& list) {
+static int write_orders(qx_handle* h, OrderCounts& oc, List&& list) {
+    std::vector<long long>* pos = oc.pos;
     cudaFree(h->d_orders);
     h->d_orders = nullptr;
     long long total = 0, most = 0;
@@ -407,9 +418,9 @@ static int write_orders(qx_handle* h, int nkey, std::vector<long long>* pos, Lis
         if (!L) return fail(QX_E_CUDA, "quartet list of a class not read back");
         const int nt = order_threads(w.nq);
         host_parallel(nt, [&](int t) {
-            long long* H = pos[c].data() + (size_t)t * nkey;
+            long long* H = pos[c].data() + (size_t)t * oc.nkey;
             for (long long q = w.nq * t / nt; q < w.nq * (t + 1) / nt; ++q)
-                order[H[seg_key(quartet_prims(h, L[q]))]++] = (int)q;
+                order[H[seg_key(oc.prims(L[q]))]++] = (int)q;
         });
         QX_CUDA(cudaMemcpy(h->d_orders + off, order.get(), sizeof(int) * w.nq, cudaMemcpyHostToDevice));
         w.d_order = h->d_orders + off;
@@ -862,6 +873,7 @@ extern "C" int qx_initialize(int natom, const double* coords, int nshell, const 
                 fn(quartet_class(h->pcls[pb], h->pcls[pk]), key(pb, pk), pb, pk);
             }
     };
+    OrderCounts oc(h);
     std::vector<long long> cnt((size_t)nt * QX_NCLS_ALL * NKEY, 0);
     std::vector<long long> tprims((size_t)nt * QX_NCLS_ALL, 0), tfull((size_t)nt * QX_NCLS_ALL, 0);
     host_parallel(nt, [&](int t) {
@@ -870,7 +882,7 @@ extern "C" int qx_initialize(int natom, const double* coords, int nshell, const 
         long long* F = tfull.data() + (size_t)t * QX_NCLS_ALL;
         visit(t, [&](int c, int k, int pb, int pk) {
             C[(size_t)c * NKEY + k]++;
-            P[c] += (long long)h->pairs[pb].nprim * h->pairs[pk].nprim;
+            P[c] += (long long)oc.nleft[pb] * oc.nleft[pk];
             F[c] += (long long)h->nfull[pb] * h->nfull[pk];
         });
     });
@@ -936,10 +948,8 @@ extern "C" int qx_initialize(int natom, const double* coords, int nshell, const 
     std::sort(h->order, h->order + QX_NCLS_ALL,
               [&](int x, int y) { return full_c[x] * g_class_nout[x] > full_c[y] * g_class_nout[y]; });
     {
-        const int nkey = order_keys(h);
-        std::vector<long long> pos[QX_NCLS_ALL];
-        for (int c = 0; c < QX_NCLS_ALL; ++c) count_order(h, c, sorted[c].get(), nkey, pos[c]);
-        const int rc = write_orders(h, nkey, pos, [&](int c) { return (const int2*)sorted[c].get(); });
+        for (int c = 0; c < QX_NCLS_ALL; ++c) count_order(h, c, sorted[c].get(), oc);
+        const int rc = write_orders(h, oc, [&](int c) { return (const int2*)sorted[c].get(); });
         if (rc) {
             free_handle(h);
             return rc;
@@ -1000,8 +1010,7 @@ extern "C" int qx_partition_costs(const double* cost, long long n, int nranks, l
 static int rebuild_views(qx_handle* h) {
     QX_CUDA(cudaDeviceSynchronize());
     const int rank = h->shard_rank, nranks = h->shard_n;
-    const int nkey = order_keys(h);
-    std::vector<long long> pos[QX_NCLS_ALL];
+    OrderCounts oc(h);
     std::vector<int2> L;
     long long base = 0;
     h->nunique = 0;
@@ -1037,10 +1046,10 @@ static int rebuild_views(qx_handle* h) {
         w.unique_base = base;
         base += w.nq * g_class_nout[c];
         h->nunique += w.nq;
-        count_order(h, c, L.data() + lo, nkey, pos[c]);
+        count_order(h, c, L.data() + lo, oc);
     }
     h->unique_size = base;
-    const int rc = write_orders(h, nkey, pos, [&](int c) -> const int2* {
+    const int rc = write_orders(h, oc, [&](int c) -> const int2* {
         const ClassWork& w = h->work[c];
         L.resize((size_t)w.nq);
         return cudaMemcpy(L.data(), w.d_q, sizeof(int2) * w.nq, cudaMemcpyDeviceToHost) == cudaSuccess ? L.data()
