@@ -248,9 +248,10 @@ int qx_set_engine(qx_handle *h, int cls, int plain, int pparam, int deriv, int d
  * without faulting the GPU. */
 int qx_set_wait_limit(qx_handle *h, int polls);
 
-/* Frees the first-derivative accumulators of the split-mode classes that a
- * handle keeps after its first derivative call (up to 512 MiB per class; the
- * next derivative call allocates them again).  No counterpart in the reference;
+/* Frees the first-derivative accumulators that a handle keeps after its first
+ * derivative call (up to 512 MiB per split-mode class, up to 64 MiB per class whose
+ * first-derivative tensor runs on the Rys engine; the next derivative call allocates
+ * them again).  No counterpart in the reference;
  * for callers that hold many handles on one device (batched SCF).  Synchronises
  * the device. */
 int qx_release_scratch(qx_handle *h);

@@ -117,6 +117,7 @@ QX_FOR_EACH_CLASS_ALL(QX_DECL_TILE)
 #undef QX_DECL_TILE
 static TileLaunch g_tile_launch[QX_NCLS_ALL];
 const double* qx_rys_table();
+void qx_launch_rys_join(const qx::RysArgs& ra, int ncomp, int nb, int nc, int nd, cudaStream_t s);
 static int g_coop_idx[QX_NCLS_ALL];
 static int g_der_idx[QX_NCLS_ALL];
 static const int g_class_nacc[QX_NCLS_ALL] = QX_CLASS_NACC;
@@ -238,6 +239,7 @@ struct ClassWork {
     // buffers; task quartet indices are relative to their slice
     std::vector<long long> slice_q, slice_t;  // quartet / task boundaries, nslice + 1 each
     double* d_pacc = nullptr;  // plain split-mode accumulators (one slice)
+    long long join_off = -1;   // this class's doubles in qx_handle::d_join (-1: none)
     // mixed precision: the full list holds its FP64 quartets first; n64_full of
     // them, nq64 in this rank's view
     long long n64_full = 0x7fffffffffffffffLL, nq64 = 0x7fffffffffffffffLL;
@@ -273,6 +275,7 @@ struct qx_handle {
     PrimPair* d_prims = nullptr;
     PairInfo* d_pairs = nullptr;
     int* d_orders = nullptr;  // the classes' processing orders
+    double* d_join = nullptr;  // parts' sums of the Rys first-derivative tensors (join_space)
     // pair records and primitive pairs with none dropped, for the second-derivative
     // programs of the s and p classes (null: nothing was dropped from their pairs); behind
     // the others in the same allocations
@@ -564,6 +567,7 @@ static void free_handle(qx_handle* h) {
     if (!h) return;
     cudaFree(h->d_prims);
     cudaFree(h->d_orders);
+    cudaFree(h->d_join);
     cudaFree(h->d_pairs);
     cudaFree(h->d_boys);
     cudaFree(h->d_err);
@@ -1010,6 +1014,8 @@ extern "C" int qx_partition_costs(const double* cost, long long n, int nranks, l
 static int rebuild_views(qx_handle* h) {
     QX_CUDA(cudaDeviceSynchronize());
     const int rank = h->shard_rank, nranks = h->shard_n;
+    cudaFree(h->d_join);
+    h->d_join = nullptr;
     OrderCounts oc(h);
     std::vector<int2> L;
     long long base = 0;
@@ -1021,6 +1027,7 @@ static int rebuild_views(qx_handle* h) {
         cudaFree(w.d_pacc);
         w.d_dtasks = nullptr;
         w.d_dacc = w.d_pacc = nullptr;
+        w.join_off = -1;
         w.ndtask = 0;
         w.slice_q.clear();
         w.slice_t.clear();
@@ -1278,9 +1285,53 @@ static int rys_unsupported(int c, const char* what) {
 
 // Work items that share a quartet's primitives in the Rys kernels: a team walks its
 // primitives one after another (thousands of them), so few quartets would leave most
-// of the GPU idle behind the largest one.  The outputs are sums of atomics either way.
+// of the GPU idle behind the largest one.  Hessian-vector products and tensors of higher
+// order are sums of atomics either way; the parts of a first-order tensor meet in order
+// (join_space).
 static int rys_parts(long long items, long long max_prims) {
     return (int)std::min(148LL * 32 / items + 1, std::max(1LL, max_prims / 4));
+}
+
+// Work items per quartet of a first-derivative tensor: their sums (twelve values per
+// component) take at most 64 MB per class.
+static int join_parts(const ClassWork& w, int c) {
+    const long long one = w.nq * 12 * g_class_nout[c] * (long long)sizeof(double);
+    return (int)std::max(1LL, std::min<long long>(rys_parts(w.nq, w.max_prims), (64LL << 20) / one));
+}
+
+// Where the class's parts leave their sums: one buffer for all classes, allocated by the
+// first such call and kept.  Null where there is no room or the stream is being captured;
+// then one team owns a quartet.
+static double* join_space(qx_handle* h, int c, cudaStream_t cs) {
+    if (h->work[c].join_off < 0) {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(cs, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        if (h->d_join) {  // planned before this class's engine was chosen
+            cudaDeviceSynchronize();
+            cudaFree(h->d_join);
+            h->d_join = nullptr;
+        }
+        long long total = 0;
+        for (int k = 0; k < QX_NCLS_ALL; ++k) {
+            ClassWork& w = h->work[k];
+            w.join_off = -1;
+            if (!w.nq || h->deriv_eng[k] != ENG_RYS) continue;
+            const int parts = join_parts(w, k);
+            if (parts == 1) continue;
+            w.join_off = total;
+            total += w.nq * parts * 12 * g_class_nout[k];
+        }
+        if (cudaMalloc((void**)&h->d_join, sizeof(double) * total) != cudaSuccess) {
+            cudaGetLastError();
+            h->d_join = nullptr;
+            for (ClassWork& w : h->work) w.join_off = -1;
+            return nullptr;
+        }
+    }
+    return h->d_join + h->work[c].join_off;
 }
 
 // Derivative tensor of order k (1..4) of one class through the Rys engine:
@@ -1300,8 +1351,16 @@ static int run_rys_derk(qx_handle* h, int c, int k, double* out, const int* nu, 
         ra.slice_k = k;
         for (int i = 0; i < k; ++i) ra.slice_nu[i] = nu[i];
     }
-    ra.parts = rys_parts(w.nq * ra.nchunk, w.max_prims);
+    if (k > 1) {
+        ra.parts = rys_parts(w.nq * ra.nchunk, w.max_prims);
+    } else if (join_parts(w, c) > 1 && (ra.partial = join_space(h, c, cs))) {
+        ra.parts = join_parts(w, c);
+    }
     if (g_rys_launch[c](ra, RK_DER1 + k - 1, w.nq * ra.nchunk * ra.parts, cs)) return rys_unsupported(c, "derivative");
+    if (ra.partial) {
+        auto nc = [&](int i) { return (g_class_l[c][i] + 1) * (g_class_l[c][i] + 2) / 2; };
+        qx_launch_rys_join(ra, g_class_nout[c], nc(1), nc(2), nc(3), cs);
+    }
     QX_CUDA(cudaGetLastError());
     return QX_OK;
 }
@@ -1935,8 +1994,8 @@ extern "C" int qx_set_engine(qx_handle* h, int cls, int plain, int pparam, int d
     return QX_OK;
 }
 
-// Frees the first-derivative split-mode accumulators the handle keeps between
-// calls (the next derivative call of the class allocates them again), for
+// Frees the first-derivative accumulators the handle keeps between calls (the split
+// modes' and join_space; the next derivative call allocates them again), for
 // callers that hold many handles on one device.
 extern "C" int qx_release_scratch(qx_handle* h) {
     if (!h) return fail(QX_E_INVALID, "qx_release_scratch: bad handle");
@@ -1945,7 +2004,10 @@ extern "C" int qx_release_scratch(qx_handle* h) {
     for (int c = 0; c < QX_NCLS_ALL; ++c) {
         cudaFree(h->work[c].d_dacc);
         h->work[c].d_dacc = nullptr;
+        h->work[c].join_off = -1;
     }
+    cudaFree(h->d_join);
+    h->d_join = nullptr;
     return QX_OK;
 }
 

@@ -164,6 +164,7 @@ struct RysArgs {
     int chunk = 1;                // multi-indices per work item
     int nchunk = 1;               // multi-index chunks per quartet
     int parts = 1;                // work items that share a quartet's primitives (and chunk)
+    double* partial = nullptr;    // order 1, parts > 1: [work item][12][component], for k_rys_join
     int slice_k = 0;              // 0: dense; else the slice's order (== k)
     int slice_nu[4] = {0, 0, 0, 0};  // the slice's sorted nuclear indices
     // first-derivative tile (RK_DER1 only): out is a (3N, tile_E) row-major
@@ -1019,6 +1020,17 @@ __global__ void __launch_bounds__(RysCls<LA, LB, LC, LD, KIND>::BS, RysCls<LA, L
                                 for (int mm = 0; mm < MG; ++mm)
                                     if (mm < mn) acc[j][mm] += rys_prod_derk<C>(O, nrb, offs[j], mops[m0 + mm]);
                     });
+                }
+                if constexpr (KIND == RK_DER1) {
+                    if (ra.partial) {
+                        double* o = ra.partial + (w * 12 + m0) * C::NCOMP;
+#pragma unroll
+                        for (int j = 0; j < NCPT; ++j)
+#pragma unroll
+                            for (int mm = 0; mm < MG; ++mm)
+                                if (tid + j * TS < C::NCOMP && mm < mn) o[(size_t)mm * C::NCOMP + tid + j * TS] = acc[j][mm];
+                        continue;
+                    }
                 }
 #pragma unroll
                 for (int j = 0; j < NCPT; ++j) {

@@ -42,15 +42,42 @@ def test_integrals(ks, engine):
         for cls, (_, b) in eng.unique_blocks().items():
             assert cls not in exact or torch.equal(b, blocks[cls]), cls
         assert engine != "rys" or torch.equal(eng.eri(), G)
-    # images of one integral; a quartet with two equal shells or pairs holds some of its
-    # images as components of their own, each with its own rounding
-    b = eng.basis
+    _images(eng.basis, G)
+
+
+def _images(b, G):
+    """The images of one integral are equal; a quartet with two equal shells or pairs holds
+    some of its images as components of their own, each with its own rounding."""
     sh = torch.cat([torch.full(((s.l + 1) * (s.l + 2) // 2,), i) for i, s in enumerate(b.shells)]).cuda()
     i, j, k, l = (sh.view([-1 if a == x else 1 for a in range(4)]) for x in range(4))
     own = (i == j) | (k == l) | ((torch.minimum(i, j) == torch.minimum(k, l)) & (torch.maximum(i, j) == torch.maximum(k, l)))
     for p in itertools.permutations(range(4)):
         if {p[0], p[1]} in ({0, 1}, {2, 3}):
             assert bool(((G.permute(p) == G) | own).all()), p
+
+
+@pytest.mark.parametrize("ks,ls", [((5,), (0, 1, 2, 3)), ((1, 8), (0, 1, 3)), ((2,), (0, 3))])
+def test_first_derivatives(ks, ls):
+    """First-derivative tensors of the Rys engine, a quartet's primitives in one and in
+    several parts: the tensor, its slices, and both after the parts' buffer was given back
+    and after it was planned anew for more classes."""
+    eng = EriEngine(_basis(ks, ls), 1e-12)
+    first = eng.eri_deriv_core(1).clone()  # f classes by the Rys engine
+    for c in eng.class_info():
+        eng.set_engine(c["cls"], deriv="rys")
+    dG = eng.eri_deriv_core(1).clone()
+    scale = dG.abs().max()
+    assert (first - dG).abs().max() < 1e-9 * max(1.0, scale.item())
+    for x in range(dG.shape[0]):
+        _images(eng.basis, dG[x])
+    for _ in range(2):
+        assert torch.equal(eng.eri_deriv_core(1), dG)
+        eng.release_scratch()
+    nu = np.zeros(dG.shape[0], dtype=int)
+    for x in (0, 4):
+        nu[:] = 0
+        nu[x] = 1
+        assert torch.equal(eng.eri_deriv(nu), dG[x])
 
 
 # atoms, how many of them carry shells: nuclei in 2, 4, 16 and 32 slices (one to eight
