@@ -27,6 +27,7 @@
 #include <new>
 #include <string>
 #include <thread>
+#include <utility>
 #include <vector>
 
 #include "quax_b200.h"
@@ -332,17 +333,15 @@ static void host_parallel(int nt, F&& f) {
 // 2^31 - 1 quartets, whose positions the entries do not hold, and a device or host without
 // room for the entries (half of the quartet list) run in list order.
 //
-// A counting sort over host threads, in two steps so that one class's list is on the host
-// at a time: thread t counts its contiguous range (count_order, which leaves every
-// thread's first position per key in `pos`), and writes it (write_orders).
-static int order_threads(long long nq) {
-    return (int)std::max<long long>(1, std::min<long long>({32, (long long)std::thread::hardware_concurrency(),
-                                                            nq / 16384}));
-}
+// A counting sort over host threads, in two steps (count_orders, write_orders) that take
+// any set of classes at a time: all of them where the lists are on the host, one by one
+// where they have to be fetched.  Thread t counts its contiguous range of every class of
+// the set, and after a scan in (key, thread) order writes it.
 struct OrderCounts {
     std::vector<int> nleft;  // primitive pairs per shell pair, apart from the records: the sort's only reads
     int nkey = 0;            // keys up to the largest quartet of the handle
-    std::vector<long long> pos[QX_NCLS_ALL];
+    std::vector<long long> pos[QX_NCLS_ALL];  // [thread][key] counts, then first positions; empty: no order
+    int nt[QX_NCLS_ALL] = {};
     explicit OrderCounts(const qx_handle* h) {
         int top = 1;
         for (const auto& p : h->pairs) {
@@ -351,83 +350,116 @@ struct OrderCounts {
         }
         nkey = seg_key((long long)top * top) + 1;
     }
-    long long prims(const int2& q) const { return (long long)nleft[q.x] * nleft[q.y]; }
+    int key(const int2& q) const { return seg_key((long long)nleft[q.x] * nleft[q.y]); }
 };
 
-static void count_order(qx_handle* h, int c, const int2* list, OrderCounts& oc) {
+static void count_orders(qx_handle* h, OrderCounts& oc, const std::vector<std::pair<int, const int2*>>& set) {
     const int nkey = oc.nkey;
-    std::vector<long long>& pos = oc.pos[c];
-    ClassWork& w = h->work[c];
-    w.d_order = nullptr;
-    w.uniform = true;
-    w.max_prims = 0;
-    if (!w.nq) return;
-    const int nt = order_threads(w.nq);
-    pos.assign((size_t)nt * nkey, 0);
-    std::vector<long long> top(nt, 0), sum(nkey, 0);
-    host_parallel(nt, [&](int t) {
-        long long* H = pos.data() + (size_t)t * nkey;
-        long long mx = 0;
-        for (long long q = w.nq * t / nt; q < w.nq * (t + 1) / nt; ++q) {
-            const long long n = oc.prims(list[q]);
-            ++H[seg_key(n)];
-            mx = std::max(mx, n);
-        }
-        top[t] = mx;
-    });
-    long long run = 0;
-    int used = 0;
-    for (int b = nkey - 1; b >= 0; --b) {  // largest first
-        const long long before = run;
-        for (int t = 0; t < nt; ++t) {
-            long long& x = pos[(size_t)t * nkey + b];
-            const long long v = x;
-            x = run;
-            run += v;
-        }
-        sum[b] = run - before;
-        used += run != before;
+    long long total = 0;
+    for (const auto& e : set) total += h->work[e.first].nq;
+    const int nt = (int)std::max(1LL, std::min<long long>({16, (long long)std::thread::hardware_concurrency(),
+                                                           total >> 15}));
+    std::vector<long long> top((size_t)nt * set.size(), 0);
+    for (const auto& e : set) {
+        oc.pos[e.first].resize((size_t)nt * nkey);
+        oc.nt[e.first] = nt;
     }
-    w.uniform = used == 1;
-    w.max_prims = *std::max_element(top.begin(), top.end());
-    seg_prefix(sum.data(), nkey, w.prefix);
-    if (w.uniform || w.nq > 0x7fffffffLL) std::vector<long long>().swap(pos);
+    host_parallel(nt, [&](int t) {
+        for (size_t k = 0; k < set.size(); ++k) {
+            const int2* list = set[k].second;
+            const long long nq = h->work[set[k].first].nq;
+            long long* H = oc.pos[set[k].first].data() + (size_t)t * nkey;
+            std::fill(H, H + nkey, 0);
+            long long mx = 0;
+            for (long long q = nq * t / nt; q < nq * (t + 1) / nt; ++q) {
+                const long long n = (long long)oc.nleft[list[q].x] * oc.nleft[list[q].y];
+                ++H[seg_key(n)];
+                mx = std::max(mx, n);
+            }
+            top[t * set.size() + k] = mx;
+        }
+    });
+    host_parallel((int)std::min<size_t>(nt, set.size()), [&](int t0) {
+        std::vector<long long> sum(nkey);
+        for (size_t k = t0; k < set.size(); k += nt) {
+            ClassWork& w = h->work[set[k].first];
+            std::vector<long long>& pos = oc.pos[set[k].first];
+            long long run = 0;
+            int used = 0;
+            for (int b = nkey - 1; b >= 0; --b) {  // largest first
+                const long long before = run;
+                for (int t = 0; t < nt; ++t) {
+                    long long& x = pos[(size_t)t * nkey + b];
+                    const long long v = x;
+                    x = run;
+                    run += v;
+                }
+                sum[b] = run - before;
+                used += run != before;
+            }
+            w.d_order = nullptr;
+            w.uniform = used <= 1;
+            w.max_prims = 0;
+            for (int t = 0; t < nt; ++t) w.max_prims = std::max(w.max_prims, top[t * set.size() + k]);
+            seg_prefix(sum.data(), nkey, w.prefix);
+            if (w.uniform || w.nq > 0x7fffffffLL) std::vector<long long>().swap(pos);
+        }
+    });
 }
 
-// list(c): class c's view on the host, valid until the next call.
+// list(c): class c's view on the host, valid until the next call, or (together) until the end.
 template <class List>
-static int write_orders(qx_handle* h, OrderCounts& oc, List&& list) {
-    std::vector<long long>* pos = oc.pos;
+static int write_orders(qx_handle* h, OrderCounts& oc, bool together, List&& list) {
     cudaFree(h->d_orders);
     h->d_orders = nullptr;
-    long long total = 0, most = 0;
+    long long total = 0, room = 1LL << 22;  // entries on the host: small classes share an upload
     for (int c = 0; c < QX_NCLS_ALL; ++c)
-        if (!pos[c].empty()) {
+        if (!oc.pos[c].empty()) {
             total += h->work[c].nq;
-            most = std::max(most, h->work[c].nq);
+            room = std::max(room, h->work[c].nq);
         }
     if (!total) return QX_OK;
-    std::unique_ptr<int[]> order(new (std::nothrow) int[(size_t)most]);
+    room = std::min(room, total);
+    std::unique_ptr<int[]> order(new (std::nothrow) int[(size_t)room]);
     if (!order || cudaMalloc((void**)&h->d_orders, sizeof(int) * total) != cudaSuccess) {
         cudaGetLastError();
         h->d_orders = nullptr;
         return QX_OK;  // list order
     }
-    long long off = 0;
-    for (int c = 0; c < QX_NCLS_ALL; ++c) {
-        if (pos[c].empty()) continue;
-        ClassWork& w = h->work[c];
-        const int2* L = list(c);
-        if (!L) return fail(QX_E_CUDA, "quartet list of a class not read back");
-        const int nt = order_threads(w.nq);
+    struct Part {
+        int c;
+        const int2* list;
+        long long off;
+    };
+    long long done = 0;
+    std::vector<Part> set;
+    for (int c = 0; c < QX_NCLS_ALL;) {
+        long long n = 0;
+        set.clear();
+        for (; c < QX_NCLS_ALL && (together || set.empty()); ++c) {
+            if (oc.pos[c].empty()) continue;
+            if (n + h->work[c].nq > room) break;
+            const int2* L = list(c);
+            if (!L) return fail(QX_E_CUDA, "quartet list of a class not read back");
+            set.push_back({c, L, n});
+            n += h->work[c].nq;
+        }
+        if (set.empty()) break;
+        int nt = 1;
+        for (const Part& p : set) nt = std::max(nt, oc.nt[p.c]);
         host_parallel(nt, [&](int t) {
-            long long* H = pos[c].data() + (size_t)t * oc.nkey;
-            for (long long q = w.nq * t / nt; q < w.nq * (t + 1) / nt; ++q)
-                order[H[seg_key(oc.prims(L[q]))]++] = (int)q;
+            for (const Part& p : set) {
+                const int m = oc.nt[p.c];
+                const long long nq = h->work[p.c].nq;
+                if (t >= m) continue;
+                long long* H = oc.pos[p.c].data() + (size_t)t * oc.nkey;
+                int* o = order.get() + p.off;
+                for (long long q = nq * t / m; q < nq * (t + 1) / m; ++q) o[H[oc.key(p.list[q])]++] = (int)q;
+            }
         });
-        QX_CUDA(cudaMemcpy(h->d_orders + off, order.get(), sizeof(int) * w.nq, cudaMemcpyHostToDevice));
-        w.d_order = h->d_orders + off;
-        off += w.nq;
+        QX_CUDA(cudaMemcpy(h->d_orders + done, order.get(), sizeof(int) * n, cudaMemcpyHostToDevice));
+        for (const Part& p : set) h->work[p.c].d_order = h->d_orders + done + p.off;
+        done += n;
     }
     return QX_OK;
 }
@@ -952,8 +984,11 @@ extern "C" int qx_initialize(int natom, const double* coords, int nshell, const 
     std::sort(h->order, h->order + QX_NCLS_ALL,
               [&](int x, int y) { return full_c[x] * g_class_nout[x] > full_c[y] * g_class_nout[y]; });
     {
-        for (int c = 0; c < QX_NCLS_ALL; ++c) count_order(h, c, sorted[c].get(), oc);
-        const int rc = write_orders(h, oc, [&](int c) { return (const int2*)sorted[c].get(); });
+        std::vector<std::pair<int, const int2*>> all;
+        for (int c = 0; c < QX_NCLS_ALL; ++c)
+            if (nq_c[c]) all.push_back({c, sorted[c].get()});
+        count_orders(h, oc, all);
+        const int rc = write_orders(h, oc, true, [&](int c) { return (const int2*)sorted[c].get(); });
         if (rc) {
             free_handle(h);
             return rc;
@@ -1053,10 +1088,11 @@ static int rebuild_views(qx_handle* h) {
         w.unique_base = base;
         base += w.nq * g_class_nout[c];
         h->nunique += w.nq;
-        count_order(h, c, L.data() + lo, oc);
+        w.d_order = nullptr;
+        if (w.nq) count_orders(h, oc, {{c, L.data() + lo}});
     }
     h->unique_size = base;
-    const int rc = write_orders(h, oc, [&](int c) -> const int2* {
+    const int rc = write_orders(h, oc, false, [&](int c) -> const int2* {
         const ClassWork& w = h->work[c];
         L.resize((size_t)w.nq);
         return cudaMemcpy(L.data(), w.d_q, sizeof(int2) * w.nq, cudaMemcpyDeviceToHost) == cudaSuccess ? L.data()

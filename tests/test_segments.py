@@ -84,14 +84,14 @@ def test_segments(seg, case, ordered):
 
 
 def test_keys(seg):
-    """Keys order counts and keep apart those at a power of two; above 4,096 they span at
-    most 1/64 of the count."""
+    """Keys order counts and keep apart those at a power of two; above 64 they span at most
+    1/64 of the count."""
     ns = sorted({max(1, (1 << k) + d) for k in range(25) for d in (-1, 0, 1)} | set(range(1, 9000, 7)))
     ns = [n for n in ns if n <= 1 << 24]
     keys = [seg.seg_key_of(n) for n in ns]
     assert keys == sorted(keys)
     for a, b, ka, kb in zip(ns, ns[1:], keys, keys[1:]):
-        assert ka < kb or (b > 4096 and b - a <= b / 64 and (a - 1).bit_length() == (b - 1).bit_length())
+        assert ka < kb or (b > 64 and b - a <= b / 64 and (a - 1).bit_length() == (b - 1).bit_length())
 
 
 def test_lanes_by_average(seg):
