@@ -80,6 +80,28 @@ def test_first_derivatives(ks, ls):
         assert torch.equal(eng.eri_deriv(nu), dG[x])
 
 
+def test_first_derivatives_under_capture():
+    """A captured tensor: before the parts' buffer exists (one team per quartet), and with it."""
+    eng = EriEngine(_basis((3,), (0, 3)), 1e-12)
+    for c in eng.class_info():
+        eng.set_engine(c["cls"], deriv="rys")
+    out = torch.empty((3 * eng.natom,) + (eng.nbf,) * 4, dtype=torch.float64, device="cuda")
+
+    def captured():
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            eng.eri_deriv_core(1, out)
+        out.fill_(7.0)
+        graph.replay()
+        torch.cuda.synchronize()
+        return out.clone()
+
+    alone = captured()
+    dG = eng.eri_deriv_core(1).clone()
+    assert (alone - dG).abs().max() < 1e-12 * max(1.0, dG.abs().max().item())
+    assert torch.equal(captured(), dG)
+
+
 # atoms, how many of them carry shells: nuclei in 2, 4, 16 and 32 slices (one to eight
 # blocks per shell pair), some of them empty, and in one slice
 @pytest.mark.parametrize("natom,carry,ls", [(2, 2, (0, 1, 2)), (3, 3, (0, 1, 2)), (12, 4, (0, 1)), (24, 3, (0, 1, 2)),
