@@ -44,7 +44,7 @@ THR = 1e-12
 # DRAM traffic of a class's dominant kernel from an ncu capture of this workload
 # (dram__bytes_read.sum + dram__bytes_write.sum), with the capture it comes from
 TRAFFIC_FROM_PROFILE = {
-    (2, 2, 2, 1): {"bytes": 29.21e6, "source": "ncu capture in profiles/k_gvrr_p19_eri10.md (split VRR kernel "
+    (2, 2, 2, 1): {"bytes": 18.44e6, "source": "ncu capture in profiles/k_gvrr_p19_eri10.md (split VRR kernel "
                                                "of the class, one launch)"},
 }
 
