@@ -411,8 +411,9 @@ def _time_ms(fn, reps=1, warm=True):
 def _tile_engines(eng, D, shard=8, view=(0, 1)):
     """Per class, the fastest derivative engine among those the plain path can also
     use (warp kernels with 1 or 4 warps per quartet, Rys), timed in adjoint mode on
-    a 1/shard cost-balanced shard of the lists, so the adjoint and the plain path
-    below run the same derivative arithmetic."""
+    a 1/shard cost-balanced shard of the lists.  Both paths below then run the same
+    warp programs; "rys" is the tile kernels for the adjoint and the table kernels for
+    the plain path."""
     import torch
 
     g = torch.zeros(3 * eng.natom, dtype=torch.float64, device="cuda")
