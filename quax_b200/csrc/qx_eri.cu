@@ -910,10 +910,13 @@ extern "C" int qx_initialize(int natom, const double* coords, int nshell, const 
             }
     };
     OrderCounts oc(h);
-    std::vector<long long> cnt((size_t)nt * QX_NCLS_ALL * NKEY, 0);
+    // 32 KB per class and thread, cleared by the thread that counts in it
+    const int ncls = *std::max_element(h->l.begin(), h->l.end()) > 2 ? QX_NCLS_ALL : QX_NUM_CLASSES;
+    std::unique_ptr<long long[]> cnt(new long long[(size_t)nt * ncls * NKEY]);
     std::vector<long long> tprims((size_t)nt * QX_NCLS_ALL, 0), tfull((size_t)nt * QX_NCLS_ALL, 0);
     host_parallel(nt, [&](int t) {
-        long long* C = cnt.data() + (size_t)t * QX_NCLS_ALL * NKEY;
+        long long* C = cnt.get() + (size_t)t * ncls * NKEY;
+        std::fill(C, C + (size_t)ncls * NKEY, 0);
         long long* P = tprims.data() + (size_t)t * QX_NCLS_ALL;
         long long* F = tfull.data() + (size_t)t * QX_NCLS_ALL;
         visit(t, [&](int c, int k, int pb, int pk) {
@@ -923,11 +926,11 @@ extern "C" int qx_initialize(int natom, const double* coords, int nshell, const 
         });
     });
     std::vector<long long> nq_c(QX_NCLS_ALL, 0), prims_c(QX_NCLS_ALL, 0), full_c(QX_NCLS_ALL, 0);
-    for (int c = 0; c < QX_NCLS_ALL; ++c) {
+    for (int c = 0; c < ncls; ++c) {
         long long run = 0;
         for (int k = 0; k < NKEY; ++k)
             for (int t = 0; t < nt; ++t) {
-                long long& x = cnt[((size_t)t * QX_NCLS_ALL + c) * NKEY + k];
+                long long& x = cnt[((size_t)t * ncls + c) * NKEY + k];
                 const long long v = x;
                 x = run;
                 run += v;
@@ -942,10 +945,10 @@ extern "C" int qx_initialize(int natom, const double* coords, int nshell, const 
     for (int c = 0; c < QX_NCLS_ALL; ++c)
         if (nq_c[c]) sorted[c].reset(new int2[(size_t)nq_c[c]]);
     host_parallel(nt, [&](int t) {
-        long long* C = cnt.data() + (size_t)t * QX_NCLS_ALL * NKEY;
+        long long* C = cnt.get() + (size_t)t * ncls * NKEY;
         visit(t, [&](int c, int k, int pb, int pk) { sorted[c][C[(size_t)c * NKEY + k]++] = make_int2(pb, pk); });
     });
-    std::vector<long long>().swap(cnt);
+    cnt.reset();
     trace.mark("quartet enumeration, sort");
     long long base = 0;
     for (int c = 0; c < QX_NCLS_ALL; ++c) {

@@ -84,6 +84,16 @@ void build_pairs(const ShellTables& t, const double* coords, double tol, std::ve
     pcls.clear();
     if (nfull) nfull->clear();
     const double cut = 1e-18 * std::min(tol, 1e-10);
+    size_t np = 0;  // primitives
+    for (int s = 0; s < nshell; ++s) np += t.nprim[s];
+    const size_t room = std::min<size_t>(np * (np + 1) / 2, 1 << 22);  // grown beyond where needed
+    prims.reserve(room);
+    if (all) all->reserve(room);
+    auto power = [](double x, int n) {
+        double v = 1.0;
+        for (int i = 0; i < n; ++i) v *= x;
+        return v;
+    };
     std::vector<std::pair<PrimPair, double>> cand;  // record and size bound
     for (int s1 = 0; s1 < nshell; ++s1)
         for (int s2 = 0; s2 <= s1; ++s2) {
@@ -124,8 +134,8 @@ void build_pairs(const ShellTables& t, const double* coords, double tol, std::ve
                     // (pi / zeta)^{3/2} times the extent of its polynomials, and times
                     // the (2 zeta)^{1/4} of a Coulomb norm
                     const double w = 1.0 / std::sqrt(r.zeta);
-                    const double size = std::fabs(r.K) * std::pow(r.zeta, -0.25) * std::pow(b / r.zeta * AB + w, pi.l1) *
-                                        std::pow(a / r.zeta * AB + w, pi.l2);
+                    const double size = std::fabs(r.K) * std::sqrt(w) * power(b / r.zeta * AB + w, pi.l1) *
+                                        power(a / r.zeta * AB + w, pi.l2);
                     best = std::max(best, size);
                     // every nuclear derivative adds at most a factor of about
                     // 2 mu AB + 2 sqrt(zeta) < 8 sqrt(zeta) down to exp(-16); beyond, the
